@@ -74,6 +74,7 @@ struct lmb_lattice {
     // nseg words) and buf[1] (next nseg), one per segment of 32 sites.
     uint32_t *pb;
     uint32_t nseg;
+    uint8_t *sites_rm;  // site types in row-major order (allocated at the first row-major call)
     unsigned long long *counts_dev;
     uint32_t counts_len;
     // Species counts of the last lmb_run_counts_async (pinned), and the
@@ -720,6 +721,7 @@ extern "C" int lmb_lattice_destroy(lmb_lattice *l)
     if (l->list) cudaFree(l->list);
     if (l->rx_sites) cudaFree(l->rx_sites);
     if (l->pb) cudaFree(l->pb);
+    if (l->sites_rm) cudaFree(l->sites_rm);
     if (l->counts_dev) cudaFree(l->counts_dev);
     if (l->counts_host) cudaFreeHost(l->counts_host);
     if (l->rs_host) cudaFreeHost(l->rs_host);
@@ -774,22 +776,18 @@ extern "C" int lmb_lattice_set_row_major(lmb_lattice *l, const void *particles, 
     lmb_ctx *c = l->ctx;
     CK(cudaSetDevice(c->device));
     const size_t pbytes = (size_t)l->g.N * l->slots * l->bps;
-    void *tmp = nullptr;
-    uint8_t *tmp_sites = nullptr;
-    CK(cudaMalloc(&tmp, pbytes));
-    cudaError_t e = cudaMalloc(&tmp_sites, l->g.N);
-    if (e == cudaSuccess) e = cudaMemcpyAsync(tmp, particles, pbytes, cudaMemcpyHostToDevice, c->stream);
-    if (e == cudaSuccess) e = cudaMemcpyAsync(tmp_sites, sites, l->g.N, cudaMemcpyHostToDevice, c->stream);
+    if (!l->sites_rm) CK(cudaMalloc(&l->sites_rm, l->g.N));
+    // The row-major particles pass through the buffer the next timestep
+    // writes: the same size, and free between runs.
+    uint32_t *tmp = l->buf[l->cur ^ 1];
+    CK(cudaMemcpyAsync(tmp, particles, pbytes, cudaMemcpyHostToDevice, c->stream));
+    CK(cudaMemcpyAsync(l->sites_rm, sites, l->g.N, cudaMemcpyHostToDevice, c->stream));
     reset_overflow_queue(l);
-    if (e == cudaSuccess) e = cudaMemcpyAsync(l->rs, l->rs_host, sizeof(RunState), cudaMemcpyHostToDevice, c->stream);
-    if (e == cudaSuccess)
-        e = launch_row_major_to_native((int)l->bps, (int)l->slots, tmp, tmp_sites, l->buf[l->cur], l->sites, l->g,
-                                       l->rs, c->stream);
-    if (e == cudaSuccess) e = cudaMemcpyAsync(l->rs_host, l->rs, sizeof(RunState), cudaMemcpyDeviceToHost, c->stream);
-    if (e == cudaSuccess) e = cudaStreamSynchronize(c->stream);
-    cudaFree(tmp);
-    if (tmp_sites) cudaFree(tmp_sites);
-    if (e != cudaSuccess) return cuda_status(e);
+    CK(cudaMemcpyAsync(l->rs, l->rs_host, sizeof(RunState), cudaMemcpyHostToDevice, c->stream));
+    CK(launch_row_major_to_native((int)l->bps, (int)l->slots, tmp, l->sites_rm, l->buf[l->cur], l->sites, l->g, l->rs,
+                                  c->stream));
+    CK(cudaMemcpyAsync(l->rs_host, l->rs, sizeof(RunState), cudaMemcpyDeviceToHost, c->stream));
+    CK(cudaStreamSynchronize(c->stream));
     // RDMESolver.cpp:160-185 rejects invalid species ids and site types.
     if (l->rs_host->max_species > number_species || l->rs_host->max_site_type >= number_site_types) {
         return LMB_E_ARG;
@@ -805,19 +803,13 @@ extern "C" int lmb_lattice_get_row_major(lmb_lattice *l, void *particles, uint8_
     lmb_ctx *c = l->ctx;
     CK(cudaSetDevice(c->device));
     const size_t pbytes = (size_t)l->g.N * l->slots * l->bps;
-    void *tmp = nullptr;
-    uint8_t *tmp_sites = nullptr;
-    CK(cudaMalloc(&tmp, pbytes));
-    cudaError_t e = sites ? cudaMalloc(&tmp_sites, l->g.N) : cudaSuccess;
-    if (e == cudaSuccess)
-        e = launch_native_to_row_major((int)l->bps, (int)l->slots, l->buf[l->cur], l->sites, tmp, tmp_sites, l->g,
-                                       c->stream);
-    if (e == cudaSuccess) e = cudaMemcpyAsync(particles, tmp, pbytes, cudaMemcpyDeviceToHost, c->stream);
-    if (e == cudaSuccess && sites) e = cudaMemcpyAsync(sites, tmp_sites, l->g.N, cudaMemcpyDeviceToHost, c->stream);
-    if (e == cudaSuccess) e = cudaStreamSynchronize(c->stream);
-    cudaFree(tmp);
-    if (tmp_sites) cudaFree(tmp_sites);
-    if (e != cudaSuccess) return cuda_status(e);
+    if (sites && !l->sites_rm) CK(cudaMalloc(&l->sites_rm, l->g.N));
+    uint32_t *tmp = l->buf[l->cur ^ 1];  // free between runs (lmb_lattice_set_row_major)
+    CK(launch_native_to_row_major((int)l->bps, (int)l->slots, l->buf[l->cur], l->sites, tmp,
+                                  sites ? l->sites_rm : nullptr, l->g, c->stream));
+    CK(cudaMemcpyAsync(particles, tmp, pbytes, cudaMemcpyDeviceToHost, c->stream));
+    if (sites) CK(cudaMemcpyAsync(sites, l->sites_rm, l->g.N, cudaMemcpyDeviceToHost, c->stream));
+    CK(cudaStreamSynchronize(c->stream));
     return LMB_OK;
 }
 
