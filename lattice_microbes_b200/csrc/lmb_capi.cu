@@ -20,6 +20,7 @@
 #include "lmb_device.cuh"
 #include "lmb_fused.h"
 #include "lmb_internal.h"
+#include "lmb_overflow.cuh"
 
 using namespace lmb;
 
@@ -87,13 +88,18 @@ struct lmb_lattice {
     // Schedule: fused tile kernel (one launch per timestep) or per-phase kernels.
     int schedule;
     TileShape tile;
+    // Particles per site when the lattice was last counted, the figure the
+    // fused plan was made for, and whether the caller left the plan to the
+    // lattice.
+    float density, plan_density;
+    bool auto_plan;
     // Captured timestep graphs, one per starting buffer parity.
     struct Graph {
         cudaGraphExec_t exec;
         const void *model;
         const void *tables;
         int schedule;
-        uint32_t Ty, Tz;
+        uint32_t Ty, Tz, list_smem;
         bool reaction;
         uint64_t kernels;
     } graph[2];
@@ -335,6 +341,8 @@ static int upload_model(lmb_model *m)
     m->dev.rx_off = (const uint32_t *)(b + off[13]);
     m->dev.rx_list = (const uint32_t *)(b + off[14]);
     m->dev.nnz = (uint32_t)m->st_sp.size();
+    m->dev.zeroth = 0;
+    for (float q : m->qp0) m->dev.zeroth |= q != 0.0f ? 1u : 0u;
     m->dev.stage_bytes = 0;
     {
         // Tables small enough to copy into shared memory per block (16-byte
@@ -631,14 +639,14 @@ extern "C" int lmb_lattice_create(lmb_ctx *c, uint32_t X, uint32_t Y, uint32_t Z
         return cuda_status(e);
     }
     l->validated = false;
-    l->schedule = LMB_SCHEDULE_FUSED;
-    if (!fused_default_shape(l->g, (int)bps, (int)slots, l->tile)) {
-        const int rc = lmb_lattice_set_schedule(l, LMB_SCHEDULE_PHASES, 0, 0);
-        if (rc != LMB_OK) {
-            lmb_lattice_destroy(l);
-            return rc;
-        }
+    l->density = l->plan_density = LIST_DEFAULT_DENSITY;
+    int rc = lmb_lattice_set_schedule(l, LMB_SCHEDULE_FUSED, 0, 0);
+    if (rc == LMB_E_UNSUPPORTED) rc = lmb_lattice_set_schedule(l, LMB_SCHEDULE_PHASES, 0, 0);
+    if (rc != LMB_OK) {
+        lmb_lattice_destroy(l);
+        return rc;
     }
+    l->auto_plan = l->schedule == LMB_SCHEDULE_FUSED;
     *out = l;
     return LMB_OK;
 }
@@ -647,25 +655,40 @@ extern "C" int lmb_lattice_create(lmb_ctx *c, uint32_t X, uint32_t Y, uint32_t Z
 // fraction of their sites; denser ones overflow it and react over every site.
 static uint32_t reaction_list_capacity(const Geometry &g) { return g.N / 8 + 4096; }
 
+// Device memory of the per-phase schedule: the reaction site list, and the
+// plane bounds.
+static int ensure_phase_buffers(lmb_lattice *l)
+{
+    if (!l->rx_sites) {
+        CK(cudaSetDevice(l->ctx->device));
+        const uint32_t cap = reaction_list_capacity(l->g);
+        CK(cudaMalloc(&l->rx_sites, (size_t)cap * 2 * sizeof(uint32_t)));
+        l->rx_cap = cap;
+    }
+    return LMB_OK;
+}
+
+// Plane bounds need segments of 32 sites that end with the x rows.
+static int ensure_plane_bounds(lmb_lattice *l)
+{
+    if (!l->pb && l->g.X % 32u == 0) {
+        CK(cudaSetDevice(l->ctx->device));
+        const uint32_t nseg = l->g.N >> PB_SHIFT;
+        CK(cudaMalloc(&l->pb, (size_t)nseg * 2 * sizeof(uint32_t)));
+        l->nseg = nseg;
+    }
+    return LMB_OK;
+}
+
 extern "C" int lmb_lattice_set_schedule(lmb_lattice *l, int schedule, uint32_t Ty, uint32_t Tz)
 {
     if (!l) return LMB_E_ARG;
     if (schedule == LMB_SCHEDULE_PHASES) {
-        if (!l->rx_sites) {
-            CK(cudaSetDevice(l->ctx->device));
-            const uint32_t cap = reaction_list_capacity(l->g);
-            CK(cudaMalloc(&l->rx_sites, (size_t)cap * 2 * sizeof(uint32_t)));
-            l->rx_cap = cap;
-        }
-        // Plane bounds need every warp of a sweep tile to hold one whole
-        // segment: x rows a multiple of 32 sites.
-        if (!l->pb && l->g.X % 32u == 0) {
-            CK(cudaSetDevice(l->ctx->device));
-            const uint32_t nseg = l->g.N >> PB_SHIFT;
-            CK(cudaMalloc(&l->pb, (size_t)nseg * 2 * sizeof(uint32_t)));
-            l->nseg = nseg;
-        }
+        int rc = ensure_phase_buffers(l);
+        if (rc == LMB_OK) rc = ensure_plane_bounds(l);
+        if (rc) return rc;
         l->schedule = schedule;
+        l->auto_plan = false;
         return LMB_OK;
     }
     if (schedule == LMB_SCHEDULE_CLUSTER) {
@@ -674,6 +697,7 @@ extern "C" int lmb_lattice_set_schedule(lmb_lattice *l, int schedule, uint32_t T
         CK(cudaSetDevice(l->ctx->device));
         if (!cluster_plan(l->g, (int)l->bps, (int)l->slots, l->cap, 8 * 1024, C, P)) return LMB_E_UNSUPPORTED;
         l->schedule = schedule;
+        l->auto_plan = false;
         return LMB_OK;
     }
     if (schedule == LMB_SCHEDULE_GRID) {
@@ -687,15 +711,22 @@ extern "C" int lmb_lattice_set_schedule(lmb_lattice *l, int schedule, uint32_t T
         if (!ok) return LMB_E_UNSUPPORTED;
         l->tile = t;
         l->schedule = schedule;
+        l->auto_plan = false;
         return LMB_OK;
     }
     if (schedule != LMB_SCHEDULE_FUSED) return LMB_E_ARG;
     TileShape t;
-    bool ok = (Ty == 0 && Tz == 0) ? fused_default_shape(l->g, (int)l->bps, (int)l->slots, t)
-                                   : fused_make_shape(l->g, (int)l->bps, (int)l->slots, Ty, Tz, t);
+    bool ok = (Ty == 0 && Tz == 0) ? fused_default_shape(l->g, (int)l->bps, (int)l->slots, t, l->density)
+                                   : fused_make_shape(l->g, (int)l->bps, (int)l->slots, Ty, Tz, t, l->density);
     if (!ok) return LMB_E_UNSUPPORTED;
+    if (t.list_smem && l->words > 2) {
+        const int rc = ensure_plane_bounds(l);
+        if (rc) return rc;
+    }
     l->tile = t;
     l->schedule = schedule;
+    l->plan_density = l->density;
+    l->auto_plan = Ty == 0 && Tz == 0;
     return LMB_OK;
 }
 
@@ -876,14 +907,54 @@ static const uint32_t GRAPH_STEPS = 32;  // even: a replay returns to the same b
 // Plane bounds of buffer b, or null when the lattice keeps none.
 static uint32_t *plane_bounds(lmb_lattice *l, int b) { return l->pb ? l->pb + (size_t)b * l->nseg : nullptr; }
 
+// The kernels that run a timestep of the lattice's schedule: the
+// particle-list kernel where its tile fits and its list entries hold the
+// model's species ids, the dense fused kernel where they do not, and the
+// per-phase kernels for PHASES and for a tile that only the particle-list
+// kernel could hold.
+enum StepKind { STEP_LIST, STEP_DENSE, STEP_PHASES };
+
+static StepKind step_kind(const lmb_lattice *l, const lmb_model *m)
+{
+    if (l->schedule != LMB_SCHEDULE_FUSED) return STEP_PHASES;
+    if (l->tile.list_smem && (l->bps == 1 || m->ns <= LIST_MAX_SPECIES)) return STEP_LIST;
+    return l->tile.dense ? STEP_DENSE : STEP_PHASES;
+}
+
+// One fused launch (list or dense form), from the current buffer.
+static cudaError_t launch_fused_step(lmb_lattice *l, const lmb_model *m, cudaStream_t st)
+{
+    uint32_t *a = l->buf[l->cur], *b = l->buf[l->cur ^ 1];
+    if (step_kind(l, m) == STEP_DENSE)
+        return launch_fused((int)l->bps, (int)l->slots, a, b, l->sites, l->g, m->dev, l->rs, l->list, l->cap, l->tile,
+                            m->nr > 0, st);
+    const bool bounds = l->pb && l->words > 2;
+    return launch_list((int)l->bps, (int)l->slots, a, b, l->sites, l->g, m->dev, l->rs, l->list, l->cap, l->tile,
+                       m->nr > 0, bounds ? plane_bounds(l, l->cur) : nullptr,
+                       bounds ? plane_bounds(l, l->cur ^ 1) : nullptr, st);
+}
+
+// Follows the lattice's particle density with the fused plan: the default
+// tile, or the list of the caller's tile.
+static void follow_density(lmb_lattice *l)
+{
+    if (l->schedule != LMB_SCHEDULE_FUSED) return;
+    if (l->density <= 1.1f * l->plan_density && l->density >= 0.4f * l->plan_density) return;
+    TileShape t;
+    if (l->auto_plan ? fused_default_shape(l->g, (int)l->bps, (int)l->slots, t, l->density)
+                     : fused_make_shape(l->g, (int)l->bps, (int)l->slots, l->tile.Ty, l->tile.Tz, t, l->density))
+        l->tile = t;
+    l->plan_density = l->density;
+}
+
 // Queues one timestep (schedule of the lattice) and flips the buffer index.
 static cudaError_t enqueue_step(lmb_lattice *l, lmb_model *m, cudaStream_t st)
 {
     const int bps = (int)l->bps, S = (int)l->slots;
     uint32_t *a = l->buf[l->cur], *b = l->buf[l->cur ^ 1];
     cudaError_t e;
-    if (l->schedule == LMB_SCHEDULE_FUSED) {
-        e = launch_fused(bps, S, a, b, l->sites, l->g, m->dev, l->rs, l->list, l->cap, l->tile, m->nr > 0, st);
+    if (step_kind(l, m) != STEP_PHASES) {
+        e = launch_fused_step(l, m, st);
         l->cur ^= 1;
         return e;
     }
@@ -906,11 +977,13 @@ static cudaError_t enqueue_step(lmb_lattice *l, lmb_model *m, cudaStream_t st)
                           st);
 }
 
-// Both buffers' plane bounds set to every plane: the start of a per-phase
-// run, whatever was written to the buffers since the last one.
-static cudaError_t reset_plane_bounds(lmb_lattice *l, cudaStream_t st)
+// Both buffers' plane bounds set to every plane: the start of a run that
+// keeps them, whatever was written to the buffers since the last one.
+static cudaError_t reset_plane_bounds(lmb_lattice *l, const lmb_model *m, cudaStream_t st)
 {
-    if (!l->pb || l->schedule != LMB_SCHEDULE_PHASES) return cudaSuccess;
+    if (!l->pb || resident_schedule(l->schedule)) return cudaSuccess;
+    const StepKind kind = step_kind(l, m);
+    if (kind == STEP_DENSE || (kind == STEP_LIST && l->words <= 2)) return cudaSuccess;
     return launch_fill_bounds(l->pb, 2 * l->nseg, l->words, st);
 }
 
@@ -922,7 +995,8 @@ static int ensure_graph(lmb_lattice *l, lmb_model *m)
 {
     lmb_lattice::Graph &gr = l->graph[l->cur];
     const bool same = gr.exec && gr.model == m && gr.tables == m->dev_block && gr.schedule == l->schedule &&
-                      gr.Ty == l->tile.Ty && gr.Tz == l->tile.Tz && gr.reaction == (m->nr > 0);
+                      gr.Ty == l->tile.Ty && gr.Tz == l->tile.Tz && gr.list_smem == l->tile.list_smem &&
+                      gr.reaction == (m->nr > 0);
     if (same) return LMB_OK;
     if (gr.exec) {
         cudaGraphExecDestroy(gr.exec);
@@ -957,6 +1031,7 @@ static int ensure_graph(lmb_lattice *l, lmb_model *m)
     gr.schedule = l->schedule;
     gr.Ty = l->tile.Ty;
     gr.Tz = l->tile.Tz;
+    gr.list_smem = l->tile.list_smem;
     gr.reaction = m->nr > 0;
     gr.kernels = captured;
     return LMB_OK;
@@ -970,12 +1045,14 @@ static int validate_for_model(lmb_lattice *l, const lmb_model *m)
         CK(cudaStreamSynchronize(c->stream));
         l->rs_host->max_species = 0;
         l->rs_host->max_site_type = 0;
+        l->rs_host->occupied = 0;
         CK(cudaMemcpyAsync(l->rs, l->rs_host, sizeof(RunState), cudaMemcpyHostToDevice, c->stream));
         CK(launch_validate((int)l->bps, (int)l->slots, l->buf[l->cur], l->sites, l->g, l->rs, c->stream));
         CK(cudaMemcpyAsync(l->rs_host, l->rs, sizeof(RunState), cudaMemcpyDeviceToHost, c->stream));
         CK(cudaStreamSynchronize(c->stream));
         l->max_species = l->rs_host->max_species;
         l->max_site_type = l->rs_host->max_site_type;
+        l->density = (float)((double)l->rs_host->occupied / l->g.N);
         l->validated = true;
     }
     // Species ids index the qp tables unchecked on the device
@@ -1008,10 +1085,16 @@ static int run_async(lmb_lattice *l, const lmb_model *mc, uint32_t seed, uint32_
     }
     int rc = device_check ? LMB_OK : validate_for_model(l, m);
     if (rc) return rc;
+    follow_density(l);
+    const StepKind kind = step_kind(l, m);
+    if (kind == STEP_PHASES && (rc = ensure_phase_buffers(l)) != LMB_OK) return rc;
     const bool counting = count_ns != ~0u;
-    // The fused kernel counts in its last launch when its work list can hold
-    // the histogram; otherwise one pass over the final lattice follows the run.
-    const bool in_kernel = counting && n > 0 && l->schedule == LMB_SCHEDULE_FUSED && count_ns + 1 <= l->tile.R;
+    // The fused kernels count in their last launch when their shared memory
+    // holds the histogram; otherwise one pass over the final lattice follows
+    // the run.
+    const bool in_kernel = counting && n > 0 && l->schedule == LMB_SCHEDULE_FUSED &&
+                           ((kind == STEP_LIST && count_ns < LIST_MAX_COUNTED) ||
+                            (kind == STEP_DENSE && count_ns + 1 <= l->tile.R));
     if (counting) {
         rc = ensure_counts_dev(l, count_ns);
         if (rc) return rc;
@@ -1031,7 +1114,7 @@ static int run_async(lmb_lattice *l, const lmb_model *mc, uint32_t seed, uint32_
         CK(launch_validate((int)l->bps, (int)l->slots, l->buf[l->cur], l->sites, l->g, l->rs, c->stream));
         CK(launch_check_contents(l->rs, m->ns, m->nst, c->stream));
     }
-    CK(reset_plane_bounds(l, c->stream));
+    CK(reset_plane_bounds(l, m, c->stream));
     l->pending_cur0 = l->cur;
     l->pending_check = device_check;
     uint32_t done = 0;
@@ -1054,9 +1137,11 @@ static int run_async(lmb_lattice *l, const lmb_model *mc, uint32_t seed, uint32_
     for (; done < n; done++) CK(enqueue_step(l, m, c->stream));
     if (counting) {
         if (!in_kernel) {
-            // After a per-phase run the current buffer's plane bounds hold:
-            // only the planes below them are read.
-            const uint32_t *pb = l->schedule == LMB_SCHEDULE_PHASES && n > 0 ? plane_bounds(l, l->cur) : nullptr;
+            // After a run that kept them the current buffer's plane bounds
+            // hold: only the planes below them are read.
+            const bool bounded = n > 0 && !resident_schedule(l->schedule) &&
+                                 (kind == STEP_PHASES || (kind == STEP_LIST && l->words > 2));
+            const uint32_t *pb = bounded ? plane_bounds(l, l->cur) : nullptr;
             CK(launch_counts((int)l->bps, (int)l->slots, l->buf[l->cur], l->g, count_ns, l->counts_dev, c->stream,
                              pb));
         }
@@ -1136,9 +1221,11 @@ extern "C" int lmb_run_wait(lmb_lattice *l, lmb_run_stats *st)
         // The device's check of the contents, kept as the host's would be.
         l->max_species = h.max_species;
         l->max_site_type = h.max_site_type;
+        l->density = (float)((double)h.occupied / l->g.N);
         l->validated = true;
         l->pending_check = false;
     }
+    if (h.list_split) l->density = std::max(l->density, l->plan_density) * 1.5f;
     if (refused) {
         // Refused before the first timestep: the lattice is where it was.
         done = 0;
@@ -1176,14 +1263,17 @@ extern "C" int lmb_run_profiled(lmb_lattice *l, const lmb_model *mc, uint32_t se
     }
     int rc = validate_for_model(l, m);
     if (rc) return rc;
+    follow_density(l);
+    const StepKind kind = step_kind(l, m);
+    if (kind == STEP_PHASES && (rc = ensure_phase_buffers(l)) != LMB_OK) return rc;
     CK(launch_begin_run(l->rs, seed, first, n, (uint32_t)mode, c->stream));
-    CK(reset_plane_bounds(l, c->stream));
+    CK(reset_plane_bounds(l, m, c->stream));
     std::vector<cudaEvent_t> ev((size_t)n * 12);
     for (auto &e : ev) CK(cudaEventCreate(&e));
     const int bps = (int)l->bps, S = (int)l->slots;
     const int cur0 = l->cur;
     const bool cluster = resident_schedule(l->schedule);
-    const bool fused = l->schedule == LMB_SCHEDULE_FUSED || cluster;
+    const bool fused = cluster || kind != STEP_PHASES;
     if (cluster && mode != LMB_OVERFLOW_CLASSIC) return LMB_E_UNSUPPORTED;
     for (uint32_t s = 0; s < n; s++) {
         uint32_t *a = l->buf[l->cur], *b = l->buf[l->cur ^ 1];
@@ -1201,8 +1291,7 @@ extern "C" int lmb_run_profiled(lmb_lattice *l, const lmb_model *mc, uint32_t se
         }
         if (fused) {
             CK(cudaEventRecord(E[10], c->stream));
-            CK(launch_fused(bps, S, a, b, l->sites, l->g, m->dev, l->rs, l->list, l->cap, l->tile, m->nr > 0,
-                            c->stream));
+            CK(launch_fused_step(l, m, c->stream));
             CK(cudaEventRecord(E[11], c->stream));
             l->cur ^= 1;
             continue;
@@ -1374,6 +1463,7 @@ struct lmb_batch {
     RunState *states_host;  // pinned
     std::vector<FusedJob> jobs_host;
     std::vector<TileShape> tiles;  // batch plan per lattice
+    bool list;  // every member runs on the particle-list kernel (otherwise all on the dense one)
     uint32_t total_tiles;
     size_t smem;
     cudaGraphExec_t graph;
@@ -1381,6 +1471,7 @@ struct lmb_batch {
     uint32_t graph_tiles;  // launch shape the graph was captured with
     uint32_t graph_jobs;
     size_t graph_smem;
+    bool graph_list;
     bool pending;
     std::vector<uint32_t> pending_first, pending_n;
     std::vector<int> cur0;
@@ -1429,34 +1520,42 @@ static int batch_reserve(lmb_batch *b, uint32_t count)
     return LMB_OK;
 }
 
-// Checks and plans a member set; fills `plan`.
+// Checks and plans a member set; fills `plan` and says whether every member
+// can run on the particle-list kernel.
 static int batch_check_members(lmb_ctx *c, uint32_t count, lmb_lattice *const *lattices,
-                               const lmb_model *const *models, int bps, int slots, std::vector<TileShape> &plan)
+                               const lmb_model *const *models, int bps, int slots, std::vector<TileShape> &plan,
+                               bool &list)
 {
     plan.resize(count);
+    list = true;
     for (uint32_t j = 0; j < count; j++) {
         lmb_lattice *l = lattices[j];
         const lmb_model *m = models[j];
         if (!l || !m || l->ctx != c || m->ctx != c) return LMB_E_ARG;
         if ((int)l->bps != bps || (int)l->slots != slots) return LMB_E_ARG;
         if (m->has_desc && (m->X != l->g.X || m->Y != l->g.Y || m->Z != l->g.Z)) return LMB_E_ARG;
-        if (!fused_batch_shape(l->g, bps, slots, plan[j])) return LMB_E_UNSUPPORTED;
+        if (list && (!fused_batch_shape(l->g, bps, slots, true, l->density, plan[j]) ||
+                     (bps != 1 && m->ns > LIST_MAX_SPECIES)))
+            list = false;
     }
+    for (uint32_t j = 0; j < count && !list; j++)
+        if (!fused_batch_shape(lattices[j]->g, bps, slots, false, 0.0f, plan[j])) return LMB_E_UNSUPPORTED;
     return LMB_OK;
 }
 
 static int batch_set(lmb_batch *b, uint32_t count, lmb_lattice *const *lattices, const lmb_model *const *models,
-                     std::vector<TileShape> &plan)
+                     std::vector<TileShape> &plan, bool list)
 {
     int rc = batch_reserve(b, count);
     if (rc) return rc;
     for (uint32_t j = 0; j < count; j++) {
         const auto it = b->tuned.find(size_key(lattices[j]->g));
         TileShape t;
-        if (it != b->tuned.end() &&
-            fused_batch_shape_ok(lattices[j]->g, b->bps, b->slots, it->second.first, it->second.second, t))
+        if (it != b->tuned.end() && fused_batch_shape_ok(lattices[j]->g, b->bps, b->slots, list, lattices[j]->density,
+                                                         it->second.first, it->second.second, t))
             plan[j] = t;
     }
+    b->list = list;
     b->lats.assign(lattices, lattices + count);
     b->models.assign(models, models + count);
     b->tiles.swap(plan);
@@ -1475,7 +1574,8 @@ extern "C" int lmb_batch_create(lmb_ctx *c, uint32_t count, lmb_lattice *const *
     *out = nullptr;
     const int bps = (int)lattices[0]->bps, slots = (int)lattices[0]->slots;
     std::vector<TileShape> plan;
-    int rc = batch_check_members(c, count, lattices, models, bps, slots, plan);
+    bool list = false;
+    int rc = batch_check_members(c, count, lattices, models, bps, slots, plan, list);
     if (rc) return rc;
     CK(cudaSetDevice(c->device));
     lmb_batch *b = new (std::nothrow) lmb_batch;
@@ -1498,7 +1598,8 @@ extern "C" int lmb_batch_create(lmb_ctx *c, uint32_t count, lmb_lattice *const *
     b->pending = false;
     b->total_tiles = 0;
     b->smem = 0;
-    rc = batch_set(b, count, lattices, models, plan);
+    b->list = b->graph_list = false;
+    rc = batch_set(b, count, lattices, models, plan, list);
     if (rc) {
         lmb_batch_destroy(b);
         return rc;
@@ -1513,10 +1614,11 @@ extern "C" int lmb_batch_set_lattices(lmb_batch *b, uint32_t count, lmb_lattice 
     if (!b || !lattices || !models || count == 0) return LMB_E_ARG;
     if (b->pending) return LMB_E_STATE;
     std::vector<TileShape> plan;
-    int rc = batch_check_members(b->ctx, count, lattices, models, b->bps, b->slots, plan);
+    bool list = false;
+    int rc = batch_check_members(b->ctx, count, lattices, models, b->bps, b->slots, plan, list);
     if (rc) return rc;
     CK(cudaSetDevice(b->ctx->device));
-    return batch_set(b, count, lattices, models, plan);
+    return batch_set(b, count, lattices, models, plan, list);
 }
 
 extern "C" int lmb_batch_destroy(lmb_batch *b)
@@ -1550,6 +1652,15 @@ static int batch_prepare(lmb_batch *b)
         }
         int rc = validate_for_model(l, m);
         if (rc) return rc;
+        if (b->list) {
+            // The list follows the lattice's density (a split tile in the
+            // last run, new contents), in the member's tile while it fits.
+            TileShape t;
+            const TileShape &p = b->tiles[j];
+            if (fused_batch_shape_ok(l->g, b->bps, b->slots, true, l->density, p.Ty, p.Tz, t) ||
+                fused_batch_shape(l->g, b->bps, b->slots, true, l->density, t))
+                b->tiles[j] = t;
+        }
         FusedJob &jb = b->jobs_host[j];
         jb.buf[0] = l->buf[0];
         jb.buf[1] = l->buf[1];
@@ -1565,7 +1676,9 @@ static int batch_prepare(lmb_batch *b)
         jb.tile_begin = tiles;
         b->cur0[j] = l->cur;
         tiles += b->tiles[j].tiles_y * b->tiles[j].tiles_z;
-        const size_t sm = fused_smem_bytes(b->tiles[j], l->g.X, l->words, l->cap, m->dev.stage_bytes);
+        const size_t sort = (size_t)pow2_at_least(l->cap) * sizeof(OverflowEntry);
+        const size_t sm = b->list ? std::max((size_t)b->tiles[j].list_smem + m->dev.stage_bytes, sort)
+                                  : fused_smem_bytes(b->tiles[j], l->g.X, l->words, l->cap, m->dev.stage_bytes);
         if (sm > smem) smem = sm;
     }
     b->total_tiles = tiles;
@@ -1579,6 +1692,14 @@ static int batch_prepare(lmb_batch *b)
 // firsts[j] + counts[j] - 1 (or first .. first + n - 1 for all when the
 // arrays are null); the launch count is the longest range, and a lattice
 // whose range is done sits out the remaining launches.
+static cudaError_t launch_batch_step(lmb_batch *b, uint32_t parity)
+{
+    const uint32_t count = (uint32_t)b->lats.size();
+    return b->list ? launch_list_batch(b->bps, b->slots, b->jobs, count, b->total_tiles, b->smem, parity, b->ctx->stream)
+                   : launch_fused_batch(b->bps, b->slots, b->jobs, count, b->total_tiles, b->smem, parity,
+                                        b->ctx->stream);
+}
+
 static int batch_run(lmb_batch *b, const uint32_t *seeds, uint32_t first, uint32_t n, const uint32_t *firsts,
                      const uint32_t *counts, int mode)
 {
@@ -1611,7 +1732,8 @@ static int batch_run(lmb_batch *b, const uint32_t *seeds, uint32_t first, uint32
         // One graph of BATCH_GRAPH_STEPS launches (parities 0, 1, ...) serves
         // every run: the job table it reads is rewritten before each run.
         static_assert(BATCH_GRAPH_STEPS % 2 == 0, "graph must return to parity 0");
-        if (b->graph && (b->graph_tiles != b->total_tiles || b->graph_smem != b->smem || b->graph_jobs != count)) {
+        if (b->graph && (b->graph_tiles != b->total_tiles || b->graph_smem != b->smem || b->graph_jobs != count ||
+                         b->graph_list != b->list)) {
             cudaGraphExecDestroy(b->graph);  // the member set or a tile plan changed
             b->graph = nullptr;
         }
@@ -1620,7 +1742,7 @@ static int batch_run(lmb_batch *b, const uint32_t *seeds, uint32_t first, uint32
             if (cudaStreamBeginCapture(c->stream, cudaStreamCaptureModeThreadLocal) == cudaSuccess) {
                 cudaError_t e = cudaSuccess;
                 for (uint32_t s = 0; s < BATCH_GRAPH_STEPS && e == cudaSuccess; s++)
-                    e = launch_fused_batch(b->bps, b->slots, b->jobs, count, b->total_tiles, b->smem, s & 1u, c->stream);
+                    e = launch_batch_step(b, s & 1u);
                 cudaGraph_t graph = nullptr;
                 const cudaError_t e2 = cudaStreamEndCapture(c->stream, &graph);
                 const uint64_t captured = lmb_kernel_launches() - l0;
@@ -1630,6 +1752,7 @@ static int batch_run(lmb_batch *b, const uint32_t *seeds, uint32_t first, uint32
                     b->graph_tiles = b->total_tiles;
                     b->graph_jobs = count;
                     b->graph_smem = b->smem;
+                    b->graph_list = b->list;
                 } else {
                     b->graph = nullptr;
                 }
@@ -1646,7 +1769,7 @@ static int batch_run(lmb_batch *b, const uint32_t *seeds, uint32_t first, uint32
         }
     }
     for (; done < launches; done++)
-        CK(launch_fused_batch(b->bps, b->slots, b->jobs, count, b->total_tiles, b->smem, done & 1u, c->stream));
+        CK(launch_batch_step(b, done & 1u));
     CK(launch_gather_states(b->rs_ptrs, count, b->states, c->stream));
     CK(cudaMemcpyAsync(b->states_host, b->states, sizeof(RunState) * count, cudaMemcpyDeviceToHost, c->stream));
     b->pending = true;
@@ -1681,6 +1804,7 @@ extern "C" int lmb_batch_wait(lmb_batch *b, lmb_run_stats *stats)
         lmb_lattice *l = b->lats[j];
         const uint32_t done = h.status == LMB_OK ? b->pending_n[j] : h.failed_step - b->pending_first[j];
         l->cur = b->cur0[j] ^ (int)((h.status == LMB_OK ? done : done + 1) & 1u);
+        if (h.list_split) l->density *= 1.5f;
         if (stats) {
             stats[j].status = h.status;
             stats[j].steps_done = done;
@@ -1775,7 +1899,7 @@ extern "C" int lmb_batch_autotune(lmb_batch *b, const uint32_t *seeds, uint32_t 
         for (uint32_t Ty : cands)
             for (uint32_t Tz : cands) {
                 TileShape t;
-                if (!fused_batch_shape_ok(g, b->bps, b->slots, Ty, Tz, t)) continue;
+                if (!fused_batch_shape_ok(g, b->bps, b->slots, b->list, b->lats[members[0]]->density, Ty, Tz, t)) continue;
                 if (t.Ty == keep.Ty && t.Tz == keep.Tz) continue;
                 for (uint32_t j : members) b->tiles[j] = t;
                 const float ms = trial();

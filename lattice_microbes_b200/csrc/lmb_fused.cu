@@ -29,6 +29,7 @@
 #include "lmb_internal.h"
 #include "lmb_overflow.cuh"
 #include "lmb_site.cuh"
+#include "lmb_stage.cuh"
 
 namespace lmb {
 
@@ -44,58 +45,6 @@ __device__ __forceinline__ void store_smem(uint32_t *buf, uint32_t R, uint32_t l
 {
 #pragma unroll
     for (int k = 0; k < SiteWords<BPS, S>::W; k++) buf[(size_t)k * R + l] = s.w[k];
-}
-
-// Copies the model tables into shared memory at `dst` (16-byte aligned;
-// stage_bytes long, each table at a 16-byte boundary) and returns a table set
-// pointing there.  The device tables sit at 256-byte boundaries of one block
-// (zero padded), so the copy moves whole 16-byte granules, every thread's
-// loads independent of each other.
-constexpr int NTABLES = 15;
-__device__ __forceinline__ DevTables stage_tables(const DevTables &m, uint8_t *dst, uint32_t tid, uint32_t nthr)
-{
-    DevTables s = m;
-    const void *srcs[NTABLES] = {m.T, m.qp0, m.qp1, m.qp2, m.order, m.D1, m.D2, m.rate, m.RL, m.stoich_off,
-                                 m.stoich_sp, m.stoich_d, m.qpmax, m.rx_off, m.rx_list};
-    const uint32_t sizes[NTABLES] = {m.nst * m.nst * m.ns * 4, m.nst * 4, m.nst * m.ns * 4,
-                                     m.nst * m.ns * m.ns * 4, m.nr * 4, m.nr * 4, m.nr * 4, m.nr * 4,
-                                     m.nr * m.nst, (m.nr + 1) * 4, m.nnz * 4, m.nnz * 4, 2 * m.nst * 4,
-                                     (m.ns + 2) * 4, m.nr * 4};
-    uint32_t first[NTABLES + 1];
-    first[0] = 0;
-#pragma unroll
-    for (int k = 0; k < NTABLES; k++) first[k + 1] = first[k] + (sizes[k] + 15u) / 16u;
-    uint4 *out = (uint4 *)dst;
-    for (uint32_t gr = tid; gr < first[NTABLES]; gr += nthr) {
-        const uint4 *src = (const uint4 *)srcs[0];
-        uint32_t f = 0;
-#pragma unroll
-        for (int j = 1; j < NTABLES; j++)
-            if (gr >= first[j]) {
-                src = (const uint4 *)srcs[j];
-                f = first[j];
-            }
-        out[gr] = __ldg(src + (gr - f));
-    }
-    const void *outs[NTABLES];
-#pragma unroll
-    for (int k = 0; k < NTABLES; k++) outs[k] = dst + 16u * first[k];
-    s.T = (const float *)outs[0];
-    s.qp0 = (const float *)outs[1];
-    s.qp1 = (const float *)outs[2];
-    s.qp2 = (const float *)outs[3];
-    s.order = (const uint32_t *)outs[4];
-    s.D1 = (const uint32_t *)outs[5];
-    s.D2 = (const uint32_t *)outs[6];
-    s.rate = (const float *)outs[7];
-    s.RL = (const uint8_t *)outs[8];
-    s.stoich_off = (const uint32_t *)outs[9];
-    s.stoich_sp = (const uint32_t *)outs[10];
-    s.stoich_d = (const int32_t *)outs[11];
-    s.qpmax = (const float *)outs[12];
-    s.rx_off = (const uint32_t *)outs[13];
-    s.rx_list = (const uint32_t *)outs[14];
-    return s;
 }
 
 template <int BPS, int S>
@@ -632,14 +581,19 @@ size_t fused_smem_bytes(const TileShape &ts, uint32_t X, uint32_t W, uint32_t ca
     return tile > sort ? tile : sort;
 }
 
-bool fused_make_shape(const Geometry &g, int bps, int slots, uint32_t Ty, uint32_t Tz, TileShape &ts)
+bool fused_make_shape(const Geometry &g, int bps, int slots, uint32_t Ty, uint32_t Tz, TileShape &ts, float density)
 {
     if (!slots_supported(bps, slots) || slots > 16) return false;  // 2-bit codes of 16 slots per word
     if (Ty == 0 || Tz == 0 || Ty > g.Y || Tz > g.Z || g.Y % Ty || g.Z % Tz) return false;
     const uint32_t W = bps == 1 ? slots / 4 : slots;
     if (g.X > 1024) return false;
     if ((Ty + 2) * (Tz + 2) > FUSED_MAX_ROWS) return false;
-    if (region_bytes(g.X, Ty, Tz, W) > FUSED_MAX_SMEM) return false;
+    ts.dense = region_bytes(g.X, Ty, Tz, W) <= FUSED_MAX_SMEM;
+    bool fits = false;
+    ts.list_smem = (uint32_t)list_smem_bytes(g, bps, slots, Ty, Tz, density, fits);
+    ts.list_fits = fits;
+    if (!ts.dense && !ts.list_smem) return false;
+    list_fill_shape(g, ts);
     ts.Ty = Ty;
     ts.Tz = Tz;
     ts.Ry = Ty + 2;
@@ -659,7 +613,7 @@ bool fused_make_shape(const Geometry &g, int bps, int slots, uint32_t Ty, uint32
 
 // Default plan: the least halo overhead among shapes that fit in shared
 // memory and still give every SM two blocks; failing that, the most blocks.
-bool fused_default_shape(const Geometry &g, int bps, int slots, TileShape &ts)
+bool fused_default_shape(const Geometry &g, int bps, int slots, TileShape &ts, float density)
 {
     const uint32_t cands[] = {1, 2, 4, 8, 16};
     bool found = false;
@@ -667,9 +621,10 @@ bool fused_default_shape(const Geometry &g, int bps, int slots, TileShape &ts)
     for (uint32_t Ty : cands)
         for (uint32_t Tz : cands) {
             TileShape t;
-            if (!fused_make_shape(g, bps, slots, Ty, Tz, t)) continue;
+            if (!fused_make_shape(g, bps, slots, Ty, Tz, t, density)) continue;
             const uint32_t W = bps == 1 ? slots / 4 : slots;
-            if (region_bytes(g.X, Ty, Tz, W) > FUSED_PREFERRED_SMEM) continue;
+            if (t.list_smem && !t.list_fits) continue;
+            if ((t.list_smem ? t.list_smem : region_bytes(g.X, Ty, Tz, W)) > FUSED_PREFERRED_SMEM) continue;
             const double tiles = (double)t.tiles_y * t.tiles_z;
             const double halo = (double)(Ty + 2) * (Tz + 2) / ((double)Ty * Tz);
             const double score = tiles >= 2 * 148 ? halo : 1e6 / tiles;
@@ -702,10 +657,12 @@ static cudaError_t ensure_smem_limit(size_t smem)
 }
 
 // A tile a batch may use: it fits, and its region leaves room for the two
-// blocks per SM the batch kernel is built for.
-bool fused_batch_shape_ok(const Geometry &g, int bps, int slots, uint32_t Ty, uint32_t Tz, TileShape &ts)
+// blocks per SM the batch kernels are built for.
+bool fused_batch_shape_ok(const Geometry &g, int bps, int slots, bool list, float density, uint32_t Ty, uint32_t Tz,
+                          TileShape &ts)
 {
-    if (!fused_make_shape(g, bps, slots, Ty, Tz, ts)) return false;
+    if (!fused_make_shape(g, bps, slots, Ty, Tz, ts, density)) return false;
+    if (list) return ts.list_fits && ts.list_smem <= FUSED_PREFERRED_SMEM;
     const uint32_t W = bps == 1 ? slots / 4 : slots;
     return region_bytes(g.X, Ty, Tz, W) <= FUSED_PREFERRED_SMEM;
 }
@@ -713,7 +670,7 @@ bool fused_batch_shape_ok(const Geometry &g, int bps, int slots, uint32_t Ty, ui
 // Batch plan: the batch already fills the GPU with many lattices, so each
 // lattice takes the tile with the least halo overhead that still lets two
 // blocks share an SM.
-bool fused_batch_shape(const Geometry &g, int bps, int slots, TileShape &ts)
+bool fused_batch_shape(const Geometry &g, int bps, int slots, bool list, float density, TileShape &ts)
 {
     const uint32_t cands[] = {1, 2, 4, 8, 16};
     bool found = false;
@@ -721,9 +678,7 @@ bool fused_batch_shape(const Geometry &g, int bps, int slots, TileShape &ts)
     for (uint32_t Ty : cands)
         for (uint32_t Tz : cands) {
             TileShape t;
-            if (!fused_make_shape(g, bps, slots, Ty, Tz, t)) continue;
-            const uint32_t W = bps == 1 ? slots / 4 : slots;
-            if (region_bytes(g.X, Ty, Tz, W) > FUSED_PREFERRED_SMEM) continue;
+            if (!fused_batch_shape_ok(g, bps, slots, list, density, Ty, Tz, t)) continue;
             const double halo = (double)(Ty + 2) * (Tz + 2) / ((double)Ty * Tz);
             const double score = halo - 1e-6 * Ty * Tz;
             if (score < best) {
@@ -1301,7 +1256,7 @@ bool fused_grid_fits(const Geometry &g, int bps, int slots, uint32_t cap, uint32
 {
     const uint32_t W = bps == 1 ? slots / 4 : slots;
     const size_t smem = fused_smem_bytes(ts, g.X, W, cap, stage_bytes);
-    if (smem > FUSED_MAX_SMEM) return false;
+    if (!ts.dense || smem > FUSED_MAX_SMEM) return false;
     return ts.tiles_y * ts.tiles_z <= grid_capacity(bps, slots, smem);
 }
 

@@ -14,6 +14,13 @@ constexpr size_t FUSED_MAX_SMEM = 200 * 1024;       // per block, below the 227 
 constexpr size_t FUSED_PREFERRED_SMEM = 100 * 1024; // default plan: two blocks per SM
 constexpr uint32_t FUSED_MAX_ROWS = 324;            // (Ty + 2) * (Tz + 2), up to 16 x 16 tiles
 
+// Particle-list form (lmb_list.cu).
+constexpr size_t LIST_MAX_SMEM = 204 * 1024;        // per block, besides the staged tables
+constexpr uint32_t LIST_MAX_COUNTED = 1024;         // entries of its species-count histogram
+constexpr uint32_t LIST_SMALL_REGION = 2048;        // regions of up to this many sites run in small blocks
+constexpr uint32_t LIST_MAX_SPECIES = 4095;         // species ids a list entry holds
+constexpr float LIST_DEFAULT_DENSITY = 0.5f;        // particles per site assumed until a lattice was counted
+
 // A block owns Ty x Tz full x-rows; its region adds one halo row on each side
 // in y and z: R = X * (Ty + 2) * (Tz + 2) sites.
 struct TileShape {
@@ -24,6 +31,10 @@ struct TileShape {
     uint32_t MW;  // 32-bit occupancy mask words per row
     uint32_t vec;  // region rows are 16-byte aligned: load them with 16-byte accesses
     uint32_t bx, by;
+    uint32_t dense;      // the dense kernel's region fits
+    uint32_t list_smem;  // shared memory of the particle-list kernel (tables excluded), 0: its region does not fit
+    uint32_t list_fits;  // its list holds the particles expected in a region
+    uint32_t magic_x, magic_q;  // its multipliers for divisions by X and X / 4
 };
 
 // One lattice of a batch run: both buffers (the run starts from buf[cur0]),
@@ -46,14 +57,34 @@ struct FusedJob {
 cudaError_t launch_fused_batch(int bytes_per_slot, int slots, const FusedJob *jobs, uint32_t njobs,
                                uint32_t total_tiles, size_t smem, uint32_t parity, cudaStream_t stream);
 
-bool fused_make_shape(const Geometry &g, int bytes_per_slot, int slots, uint32_t Ty, uint32_t Tz, TileShape &ts);
-bool fused_default_shape(const Geometry &g, int bytes_per_slot, int slots, TileShape &ts);
-bool fused_batch_shape(const Geometry &g, int bytes_per_slot, int slots, TileShape &ts);
-bool fused_batch_shape_ok(const Geometry &g, int bytes_per_slot, int slots, uint32_t Ty, uint32_t Tz, TileShape &ts);
+// density: particles per site the list of a particle-list tile is sized for.
+bool fused_make_shape(const Geometry &g, int bytes_per_slot, int slots, uint32_t Ty, uint32_t Tz, TileShape &ts,
+                      float density = LIST_DEFAULT_DENSITY);
+bool fused_default_shape(const Geometry &g, int bytes_per_slot, int slots, TileShape &ts,
+                         float density = LIST_DEFAULT_DENSITY);
+// list: for the particle-list batch kernel, otherwise for the dense one.
+bool fused_batch_shape(const Geometry &g, int bytes_per_slot, int slots, bool list, float density, TileShape &ts);
+bool fused_batch_shape_ok(const Geometry &g, int bytes_per_slot, int slots, bool list, float density, uint32_t Ty,
+                          uint32_t Tz, TileShape &ts);
 size_t fused_smem_bytes(const TileShape &ts, uint32_t X, uint32_t W, uint32_t cap, uint32_t stage_bytes);
 cudaError_t launch_fused(int bytes_per_slot, int slots, const uint32_t *src, uint32_t *dst, const uint8_t *sites,
                          const Geometry &g, const DevTables &m, RunState *rs, OverflowEntry *list, uint32_t cap,
                          const TileShape &ts, int with_reaction, cudaStream_t stream);
+
+// Particle-list form of the same timestep (lmb_list.cu): the same tiles, the
+// particles in a shared-memory list.  list_smem_bytes: shared memory of a
+// tile (0 when its region does not fit; `fits`: with room for the particles
+// expected of it); list_fill_shape: a shape's multipliers.
+// pb_src / pb_dst: the plane bounds of the buffers (null: none kept).
+size_t list_smem_bytes(const Geometry &g, int bytes_per_slot, int slots, uint32_t Ty, uint32_t Tz, float density,
+                       bool &fits);
+void list_fill_shape(const Geometry &g, TileShape &ts);
+cudaError_t launch_list(int bytes_per_slot, int slots, const uint32_t *src, uint32_t *dst, const uint8_t *sites,
+                        const Geometry &g, const DevTables &m, RunState *rs, OverflowEntry *queue, uint32_t cap,
+                        const TileShape &ts, int with_reaction, const uint32_t *pb_src, uint32_t *pb_dst,
+                        cudaStream_t stream);
+cudaError_t launch_list_batch(int bytes_per_slot, int slots, const FusedJob *jobs, uint32_t njobs,
+                              uint32_t total_tiles, size_t smem, uint32_t parity, cudaStream_t stream);
 
 // Cluster-resident runs of small lattices (lmb_fused.cu): the whole lattice
 // in the shared memory of one thread-block cluster of C CTAs (P = Z / C z

@@ -54,6 +54,7 @@ struct DevTables {
     const int32_t *stoich_d;     // stoichiometric change
     uint32_t nnz;                // entries of the sparse stoichiometry
     uint32_t stage_bytes;        // shared-memory copy size of all tables, 0 if too large to stage
+    uint32_t zeroth;             // some site type has a nonzero zeroth-order propensity
     const float *qpmax;          // [nst] largest qp1 entry, then [nst] largest qp2 entry, per site type
     // Reactions a site can fire, by first reactant: [rx_off[0], rx_off[1])
     // lists the zeroth-order reactions, [rx_off[s], rx_off[s+1]) those whose
@@ -87,8 +88,10 @@ struct RunState {
     unsigned long long reactions;
     uint32_t max_species; // validation scratch
     uint32_t max_site_type;
+    unsigned long long occupied;  // validation: particles in the lattice
     uint32_t tiles_done;  // fused kernel: blocks finished in this launch
     uint32_t rx_count;    // per-phase schedule: sites the z sweep listed for the reaction step
+    uint32_t list_split;  // particle-list kernel: a tile of this run had more particles than its list holds
     uint32_t rx_skip;     // timesteps left to run without the list (it overflowed recently)
     // timestep_hash(seed, step, k) for the sub-steps k = 0..3 of `step`, set
     // with every change of step (the per-phase kernels read them here).

@@ -1,0 +1,108 @@
+"""The particle-list timestep kernel at the sizes where it can go wrong:
+region edges and ragged rows, tiles split because their particles do not fit
+the list, more reaction candidates than its list holds, species ids past a
+list entry's, and the species counts taken in it.  Everything is compared bit
+for bit with the oracle."""
+import numpy as np
+import pytest
+
+from lattice_microbes_b200 import configs
+from tests.cases import oracle_tables
+from tests.oracle_lib import oracle_counts, oracle_run
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.fixture(scope="module")
+def ctx(gpu):
+    from lattice_microbes_b200.solver import Context
+    c = Context(0)
+    yield c
+    c.close()
+
+
+def _run(ctx, spec, n, tile=(0, 0), lattice=None, records=1, tables=None):
+    from lattice_microbes_b200 import _lib as L
+    from lattice_microbes_b200.solver import Lattice, Model
+    t = tables or oracle_tables(spec)
+    src = spec.lattice if lattice is None else lattice
+    model = Model.from_tables(ctx, t)
+    lat = Lattice(ctx, spec.X, spec.Y, spec.Z, spec.slots, spec.bytes_per_slot)
+    lat.set_schedule(L.LMB_SCHEDULE_FUSED, *tile)
+    lat.set_native(src, spec.sites)
+    step, rc = 0, 0
+    for _ in range(records):
+        rc, st, counts = lat.run_counts(model, 11, step, n, spec.ns, check=False)
+        step += n
+        if rc:
+            break
+    out, _ = lat.get_native()
+    ref, rc_ref, st_ref = oracle_run(t, src, spec.sites, 11, 0, n * records)
+    assert rc == rc_ref
+    assert np.array_equal(out, ref)
+    if rc == 0:
+        assert np.array_equal(counts, oracle_counts(t, ref))
+    lat.close()
+    model.close()
+    return st_ref
+
+
+VARIANTS = [(4, 1), (8, 1), (16, 1), (4, 4), (8, 4), (16, 4)]
+
+
+@pytest.mark.parametrize("slots,bps", VARIANTS)
+@pytest.mark.parametrize("shape,tile", [((1, 6, 4), (2, 2)), ((2, 3, 5), (3, 1)), ((3, 1, 8), (1, 4)),
+                                        ((4, 4, 4), (4, 4)), ((12, 16, 1), (16, 1)), ((30, 6, 9), (3, 3)),
+                                        ((36, 10, 6), (5, 2)), ((48, 16, 16), (16, 4)), ((64, 8, 12), (4, 6)),
+                                        ((160, 6, 6), (2, 3))])
+def test_regions_vs_oracle(ctx, shape, tile, slots, bps):
+    spec = configs.random_problem(sum(shape) + slots, X=shape[0], Y=shape[1], Z=shape[2], slots=slots,
+                                  bytes_per_slot=bps, density=0.15 * slots, zeroth=slots == 8)
+    _run(ctx, spec, 5, tile, records=2)
+
+
+@pytest.mark.parametrize("slots,bps", VARIANTS)
+def test_crowded_corner_splits_its_tile(ctx, slots, bps):
+    """Every particle of the lattice in one corner, sites full: the mean
+    density sizes a list far too short for that corner's tile."""
+    spec = configs.random_problem(5 + slots, X=64, Y=48, Z=32, slots=slots, bytes_per_slot=bps, density=0.02,
+                                  zeroth=False)
+    N = spec.X * spec.Y * spec.Z
+    rng = np.random.default_rng(3)
+    z, y, x = np.meshgrid(np.arange(10), np.arange(14), np.arange(64), indexing="ij")
+    at = (x + y * spec.X + z * spec.X * spec.Y).reshape(-1)
+    lat = np.zeros_like(spec.lattice)
+    for k in range(slots - 1):  # one slot free: the first timesteps overflow only a little
+        sp = rng.integers(1, spec.ns + 1, at.size).astype(np.uint32)
+        here = rng.random(at.size) < (0.9 if k < slots // 2 else 0.35)
+        if bps == 1:
+            lat[(k // 4) * N + at[here]] |= sp[here] << np.uint32(8 * (k % 4))
+        else:
+            lat[k * N + at[here]] = sp[here]
+    _run(ctx, spec, 3, lattice=lat, records=2)
+
+
+@pytest.mark.parametrize("slots,bps", [(8, 1), (16, 4)])
+def test_more_reaction_candidates_than_listed(ctx, slots, bps):
+    """Rates so high that most occupied sites may react in a timestep."""
+    spec = configs.random_problem(21, X=64, Y=16, Z=16, slots=slots, bytes_per_slot=bps, density=1.2, zeroth=False)
+    spec.K = spec.K * 40.0
+    st = _run(ctx, spec, 4, (16, 8))
+    assert st.reactions > 4 * 512
+
+
+@pytest.mark.parametrize("X,slots", [(32, 8), (128, 16)])
+def test_species_past_a_list_entry(ctx, X, slots):
+    """Species ids above 4095: the dense kernel, or the per-phase kernels
+    where only the particle-list kernel could hold the tile."""
+    spec = configs.random_problem(31, X=X, Y=8, Z=8, slots=slots, bytes_per_slot=4, ns=3, nst=2, nr=3, density=0.4,
+                                  zeroth=False)
+    # The three species renamed to ids up to 5000.
+    ids = np.array([0, 17, 4097, 5000], dtype=np.uint32)
+    big = configs.ModelSpec(**{**spec.__dict__, "ns": 5000,
+                               "S": np.zeros((5000, spec.nr), np.int32), "D": np.zeros((5000, spec.nr), np.uint32),
+                               "DF": np.zeros((2, 2, 5000)), "lattice": ids[spec.lattice]})
+    for s in range(3):
+        big.S[ids[s + 1] - 1], big.D[ids[s + 1] - 1] = spec.S[s], spec.D[s]
+        big.DF[:, :, ids[s + 1] - 1] = spec.DF[:, :, s]
+    _run(ctx, big, 3, (4, 4) if X == 128 else (2, 2))
