@@ -857,6 +857,8 @@ int lmb::lattice_view(const lmb_lattice *l, LatticeView *v)
     return LMB_OK;
 }
 
+bool lmb::lattice_by_particle(const lmb_lattice *l) { return l->schedule == LMB_SCHEDULE_FUSED && l->tile.list_smem != 0; }
+
 extern "C" int lmb_lattice_device_buffers(lmb_lattice *l, void **particles, void **sites)
 {
     if (!l) return LMB_E_ARG;
@@ -939,7 +941,7 @@ static cudaError_t launch_fused_step(lmb_lattice *l, const lmb_model *m, cudaStr
 static void follow_density(lmb_lattice *l)
 {
     if (l->schedule != LMB_SCHEDULE_FUSED) return;
-    if (l->density <= 1.1f * l->plan_density && l->density >= 0.4f * l->plan_density) return;
+    if (l->density <= 1.02f * l->plan_density && l->density >= 0.8f * l->plan_density) return;
     TileShape t;
     if (l->auto_plan ? fused_default_shape(l->g, (int)l->bps, (int)l->slots, t, l->density)
                      : fused_make_shape(l->g, (int)l->bps, (int)l->slots, l->tile.Ty, l->tile.Tz, t, l->density))
@@ -1225,7 +1227,10 @@ extern "C" int lmb_run_wait(lmb_lattice *l, lmb_run_stats *st)
         l->validated = true;
         l->pending_check = false;
     }
-    if (h.list_split) l->density = std::max(l->density, l->plan_density) * 1.5f;
+    // Tiles split here and there cost little; a list too short for one tile
+    // in eight is sized anew.
+    if ((uint64_t)h.list_split * 8u > (uint64_t)l->pending_n * l->tile.tiles_y * l->tile.tiles_z)
+        l->density = std::max(l->density, l->plan_density) * 1.5f;
     if (refused) {
         // Refused before the first timestep: the lattice is where it was.
         done = 0;
@@ -1378,14 +1383,27 @@ extern "C" int lmb_lattice_autotune(lmb_lattice *l, const lmb_model *m, uint32_t
     const int cur0 = l->cur;
     const int sched0 = l->schedule;
     const TileShape tile0 = l->tile;
+    const bool auto0 = l->auto_plan;
     struct Cand { int sched; uint32_t ty, tz; };
     std::vector<Cand> cands = {{LMB_SCHEDULE_PHASES, 0, 0}, {LMB_SCHEDULE_CLUSTER, 0, 0}};
-    const uint32_t dims[] = {1, 2, 4, 8, 16};
-    for (uint32_t ty : dims)
-        for (uint32_t tz : dims) {
-            TileShape t;
-            if (fused_make_shape(l->g, (int)l->bps, (int)l->slots, ty, tz, t)) cands.push_back({LMB_SCHEDULE_FUSED, ty, tz});
-        }
+    // Fused: the eight particle-list tiles with the best estimates; every
+    // dense tile where no particle-list one fits.
+    int rc = validate_for_model(l, m);
+    if (rc != LMB_OK) {
+        cudaFree(save);
+        return rc;
+    }
+    for (const TileShape &t : list_shapes(l->g, (int)l->bps, (int)l->slots, l->density, 8))
+        cands.push_back({LMB_SCHEDULE_FUSED, t.Ty, t.Tz});
+    if (cands.size() == 2) {
+        const uint32_t dims[] = {1, 2, 4, 8, 16};
+        for (uint32_t ty : dims)
+            for (uint32_t tz : dims) {
+                TileShape t;
+                if (fused_make_shape(l->g, (int)l->bps, (int)l->slots, ty, tz, t))
+                    cands.push_back({LMB_SCHEDULE_FUSED, ty, tz});
+            }
+    }
     // LMB_SCHEDULE_GRID is not a candidate: on one lattice it times as its
     // fused plan does, and its cooperative launch cannot overlap another
     // lattice's run on a second stream, as fused launches do.
@@ -1394,7 +1412,6 @@ extern "C" int lmb_lattice_autotune(lmb_lattice *l, const lmb_model *m, uint32_t
     cudaEventCreate(&e1);
     float best = 1e30f;
     Cand bestc = {sched0, tile0.Ty, tile0.Tz};
-    int rc = LMB_OK;
     for (const Cand &cd : cands) {
         if (lmb_lattice_set_schedule(l, cd.sched, cd.ty, cd.tz) != LMB_OK) continue;
         // warm-up launch, then the timed one, each from the saved state
@@ -1432,6 +1449,7 @@ extern "C" int lmb_lattice_autotune(lmb_lattice *l, const lmb_model *m, uint32_t
     if (rc != LMB_OK) {
         l->schedule = sched0;
         l->tile = tile0;
+        l->auto_plan = auto0;
         return rc;
     }
     lmb_lattice_set_schedule(l, bestc.sched, bestc.ty, bestc.tz);
@@ -1804,7 +1822,8 @@ extern "C" int lmb_batch_wait(lmb_batch *b, lmb_run_stats *stats)
         lmb_lattice *l = b->lats[j];
         const uint32_t done = h.status == LMB_OK ? b->pending_n[j] : h.failed_step - b->pending_first[j];
         l->cur = b->cur0[j] ^ (int)((h.status == LMB_OK ? done : done + 1) & 1u);
-        if (h.list_split) l->density *= 1.5f;
+        if ((uint64_t)h.list_split * 8u > (uint64_t)b->pending_n[j] * b->tiles[j].tiles_y * b->tiles[j].tiles_z)
+            l->density *= 1.5f;
         if (stats) {
             stats[j].status = h.status;
             stats[j].steps_done = done;

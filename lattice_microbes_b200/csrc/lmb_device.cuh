@@ -238,7 +238,7 @@ struct TRow {
 __device__ __forceinline__ void push_overflow(RunState *rs, OverflowEntry *list, uint32_t cap,
                                               uint32_t phase, uint32_t site, uint32_t seq, uint32_t particle)
 {
-    uint32_t idx = atomicAdd(&rs->ovf_count, 1u);
+    const uint32_t idx = (uint32_t)(atomicAdd(run_word(rs), 1ull << 32) >> 32);
     if (idx < cap) {
         OverflowEntry e;
         e.key = ((unsigned long long)phase << KEY_PHASE_SHIFT) |

@@ -21,7 +21,10 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include <algorithm>
 #include <type_traits>
+#include <utility>
+#include <vector>
 
 #include "lmb.h"
 #include "lmb_device.cuh"
@@ -511,7 +514,7 @@ __device__ __forceinline__ void fused_tile(const uint32_t *__restrict__ src, uin
     __syncthreads();
     if (tid == 0) {
         __threadfence();
-        const uint32_t prev = atomicAdd(&rs->tiles_done, 1u);
+        const uint32_t prev = (uint32_t)atomicAdd(run_word(rs), 1ull);
         s_last = prev == ntiles - 1;
     }
     __syncthreads();
@@ -611,10 +614,35 @@ bool fused_make_shape(const Geometry &g, int bps, int slots, uint32_t Ty, uint32
     return true;
 }
 
-// Default plan: the least halo overhead among shapes that fit in shared
-// memory and still give every SM two blocks; failing that, the most blocks.
+// Tile edges considered for particle-list tiles: the divisors among them let
+// edges such as 60, 72 or 96 be cut into as many tiles as are resident.
+static const uint32_t LIST_EDGES[] = {1, 2, 3, 4, 5, 6, 7, 8, 9, 10, 12, 14, 16};
+
+std::vector<TileShape> list_shapes(const Geometry &g, int bps, int slots, float density, size_t most)
+{
+    std::vector<std::pair<double, TileShape>> found;
+    for (uint32_t Ty : LIST_EDGES)
+        for (uint32_t Tz : LIST_EDGES) {
+            TileShape t;
+            if (!fused_make_shape(g, bps, slots, Ty, Tz, t, density) || !t.list_fits) continue;
+            found.push_back({list_cost(t.tiles_y * t.tiles_z, t.R, t.list_smem, density), t});
+        }
+    std::stable_sort(found.begin(), found.end(), [](const auto &a, const auto &b) { return a.first < b.first; });
+    std::vector<TileShape> out;
+    for (size_t j = 0; j < found.size() && j < most; j++) out.push_back(found[j].second);
+    return out;
+}
+
+// Default plan: the cheapest particle-list tile; where none fits, the dense
+// tile with the least halo overhead among those that still give every SM two
+// blocks, failing that, the most blocks.
 bool fused_default_shape(const Geometry &g, int bps, int slots, TileShape &ts, float density)
 {
+    const std::vector<TileShape> list = list_shapes(g, bps, slots, density, 1);
+    if (!list.empty()) {
+        ts = list[0];
+        return true;
+    }
     const uint32_t cands[] = {1, 2, 4, 8, 16};
     bool found = false;
     double best = 1e30;
@@ -623,8 +651,7 @@ bool fused_default_shape(const Geometry &g, int bps, int slots, TileShape &ts, f
             TileShape t;
             if (!fused_make_shape(g, bps, slots, Ty, Tz, t, density)) continue;
             const uint32_t W = bps == 1 ? slots / 4 : slots;
-            if (t.list_smem && !t.list_fits) continue;
-            if ((t.list_smem ? t.list_smem : region_bytes(g.X, Ty, Tz, W)) > FUSED_PREFERRED_SMEM) continue;
+            if (region_bytes(g.X, Ty, Tz, W) > FUSED_PREFERRED_SMEM) continue;
             const double tiles = (double)t.tiles_y * t.tiles_z;
             const double halo = (double)(Ty + 2) * (Tz + 2) / ((double)Ty * Tz);
             const double score = tiles >= 2 * 148 ? halo : 1e6 / tiles;
@@ -662,25 +689,27 @@ bool fused_batch_shape_ok(const Geometry &g, int bps, int slots, bool list, floa
                           TileShape &ts)
 {
     if (!fused_make_shape(g, bps, slots, Ty, Tz, ts, density)) return false;
-    if (list) return ts.list_fits && ts.list_smem <= FUSED_PREFERRED_SMEM;
+    if (list) return ts.list_fits && ts.list_smem <= LIST_BATCH_SMEM;
     const uint32_t W = bps == 1 ? slots / 4 : slots;
     return region_bytes(g.X, Ty, Tz, W) <= FUSED_PREFERRED_SMEM;
 }
 
 // Batch plan: the batch already fills the GPU with many lattices, so each
-// lattice takes the tile with the least halo overhead that still lets two
-// blocks share an SM.
+// lattice takes the tile that still lets two blocks share an SM with the
+// least work per owned site (particle-list tiles: the estimate's
+// instructions), or the least halo overhead (dense ones).
 bool fused_batch_shape(const Geometry &g, int bps, int slots, bool list, float density, TileShape &ts)
 {
-    const uint32_t cands[] = {1, 2, 4, 8, 16};
     bool found = false;
     double best = 1e30;
-    for (uint32_t Ty : cands)
-        for (uint32_t Tz : cands) {
+    for (uint32_t Ty : LIST_EDGES)
+        for (uint32_t Tz : LIST_EDGES) {
             TileShape t;
+            if (!list && ((Ty & (Ty - 1u)) || (Tz & (Tz - 1u)))) continue;
             if (!fused_batch_shape_ok(g, bps, slots, list, density, Ty, Tz, t)) continue;
             const double halo = (double)(Ty + 2) * (Tz + 2) / ((double)Ty * Tz);
-            const double score = halo - 1e-6 * Ty * Tz;
+            const double score = list ? list_cost(296u, t.R, t.list_smem, density) / ((double)g.X * Ty * Tz)
+                                      : halo - 1e-6 * Ty * Tz;
             if (score < best) {
                 best = score;
                 ts = t;

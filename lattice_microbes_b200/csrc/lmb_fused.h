@@ -5,6 +5,8 @@
 #include <stddef.h>
 #include <stdint.h>
 
+#include <vector>
+
 #include "lmb_internal.h"
 
 namespace lmb {
@@ -16,6 +18,7 @@ constexpr uint32_t FUSED_MAX_ROWS = 324;            // (Ty + 2) * (Tz + 2), up t
 
 // Particle-list form (lmb_list.cu).
 constexpr size_t LIST_MAX_SMEM = 204 * 1024;        // per block, besides the staged tables
+constexpr size_t LIST_BATCH_SMEM = 100 * 1024;      // in a batch: two blocks per SM, the tables included
 constexpr uint32_t LIST_MAX_COUNTED = 1024;         // entries of its species-count histogram
 constexpr uint32_t LIST_SMALL_REGION = 2048;        // regions of up to this many sites run in small blocks
 constexpr uint32_t LIST_MAX_SPECIES = 4095;         // species ids a list entry holds
@@ -79,6 +82,11 @@ cudaError_t launch_fused(int bytes_per_slot, int slots, const uint32_t *src, uin
 size_t list_smem_bytes(const Geometry &g, int bytes_per_slot, int slots, uint32_t Ty, uint32_t Tz, float density,
                        bool &fits);
 void list_fill_shape(const Geometry &g, TileShape &ts);
+// Estimated SM cycles of a timestep with `tiles` tiles of R region sites.
+double list_cost(uint32_t tiles, uint32_t R, size_t smem, float density);
+// The particle-list tiles of a lattice, cheapest estimate first (at most
+// `most` of them).
+std::vector<TileShape> list_shapes(const Geometry &g, int bytes_per_slot, int slots, float density, size_t most);
 cudaError_t launch_list(int bytes_per_slot, int slots, const uint32_t *src, uint32_t *dst, const uint8_t *sites,
                         const Geometry &g, const DevTables &m, RunState *rs, OverflowEntry *queue, uint32_t cap,
                         const TileShape &ts, int with_reaction, const uint32_t *pb_src, uint32_t *pb_dst,

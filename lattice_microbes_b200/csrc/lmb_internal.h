@@ -81,7 +81,6 @@ struct RunState {
     uint32_t end_step;    // exclusive end of the current run
     int32_t status;       // LMB_OK or the error that stopped the run
     uint32_t failed_step;
-    uint32_t ovf_count;   // entries in the list, carried ones first
     uint32_t carried;     // relaxed handler: entries kept from earlier steps
     uint32_t mode;        // LMB_OVERFLOW_*
     unsigned long long overflows;
@@ -89,9 +88,12 @@ struct RunState {
     uint32_t max_species; // validation scratch
     uint32_t max_site_type;
     unsigned long long occupied;  // validation: particles in the lattice
-    uint32_t tiles_done;  // fused kernel: blocks finished in this launch
+    // One 64-bit word, so that the count of finished blocks brings the queue
+    // length with it (run_word).
+    alignas(8) uint32_t tiles_done;  // fused kernels: blocks finished in this launch
+    uint32_t ovf_count;              // entries in the overflow list, carried ones first
     uint32_t rx_count;    // per-phase schedule: sites the z sweep listed for the reaction step
-    uint32_t list_split;  // particle-list kernel: a tile of this run had more particles than its list holds
+    uint32_t list_split;  // particle-list kernel: times a tile of this run had more particles than its list holds
     uint32_t rx_skip;     // timesteps left to run without the list (it overflowed recently)
     // timestep_hash(seed, step, k) for the sub-steps k = 0..3 of `step`, set
     // with every change of step (the per-phase kernels read them here).
@@ -110,6 +112,13 @@ struct RunState {
     uint32_t grid_full[3];
 };
 
+
+// tiles_done | ovf_count << 32, for 64-bit atomics (every kernel adds to
+// either half through it).
+__host__ __device__ inline unsigned long long *run_word(RunState *rs)
+{
+    return reinterpret_cast<unsigned long long *>(&rs->tiles_done);
+}
 
 // Plane bounds (per-phase schedule, lattices whose X is a multiple of 32):
 // for each segment of 32 consecutive sites (site i in segment i >> PB_SHIFT),
@@ -207,5 +216,8 @@ struct LatticeView {
     bool pending;  // an asynchronous run is in flight
 };
 int lattice_view(const lmb_lattice *lattice, LatticeView *view);
+
+// The lattice's fused plan is one of particle-list tiles.
+bool lattice_by_particle(const lmb_lattice *lattice);
 
 }  // namespace lmb

@@ -12,6 +12,7 @@
 #include "lmb.h"
 #include "lmb_device.cuh"
 #include "lmb_internal.h"
+#include "lmb_site.cuh"
 
 namespace lmb {
 
@@ -20,19 +21,6 @@ __device__ __forceinline__ void load_site_cg(const uint32_t *lat, uint32_t N, ui
 {
 #pragma unroll
     for (int k = 0; k < SiteWords<BPS, S>::W; k++) s.w[k] = __ldcg(lat + (size_t)k * N + i);
-}
-
-// Slots up to the first empty one (ByteLattice.cpp:187-206).
-template <int BPS, int S>
-__device__ uint32_t occupancy_at(const uint32_t *lat, uint32_t N, uint32_t i)
-{
-    SiteWords<BPS, S> s;
-    load_site_cg<BPS, S>(lat, N, i, s);
-    uint32_t k = 0;
-#pragma unroll
-    for (int j = 0; j < S; j++)
-        if (k == (uint32_t)j && s.slot(j) != 0) k++;
-    return k;
 }
 
 // Raises the plane bound of site i's segment to cover slot k (pb may be
@@ -64,33 +52,67 @@ __device__ bool add_particle(uint32_t *lat, uint32_t N, uint32_t i, uint32_t p, 
     return false;
 }
 
-// Classic reinsertion (MpdRdmeSolver.cu:1113-1156): shells of radius 0..4
-// from Lattice::getNearbySites (Lattice.cpp:106-128: clamped to the lattice,
-// x outer, y, z inner), first site of the same type with a free slot.
+// A site has room exactly when its last slot is empty: resolution follows
+// the sweeps, which leave every site packed (occupied slots first), and so do
+// the reaction step and the insertions made here.
 template <int BPS, int S>
-__device__ bool reinsert_classic(uint32_t *lat, const uint8_t *sites, const Geometry &g, uint32_t idx, uint32_t p,
-                                 uint32_t *pb)
+__device__ __forceinline__ bool has_room(const uint32_t *lat, uint32_t N, uint32_t i)
 {
-    const uint32_t xc = idx % g.X, yc = (idx / g.X) % g.Y, zc = idx / g.XY;
-    const uint8_t tc = sites[idx];
-    for (uint32_t radius = 0; radius <= 4; radius++) {
-        const uint32_t mind = radius > 0 ? radius - 1 : 0, maxd = radius;
-        const double min2 = (double)(mind * mind), max2 = (double)(maxd * maxd);
+    const uint32_t last = __ldcg(lat + (size_t)(SiteWords<BPS, S>::W - 1) * N + i);
+    return BPS == 1 ? (last >> 24) == 0u : last == 0u;
+}
+
+constexpr uint32_t NO_SITE = ~0u;
+
+// Target of a classic reinsertion (MpdRdmeSolver.cu:1113-1156): shells of
+// radius 0..4 from Lattice::getNearbySites (Lattice.cpp:106-128: clamped to
+// the lattice, x outer, y, z inner), first site of the same type with a free
+// slot; NO_SITE when there is none.  The site itself and its six neighbours
+// (radius 0 and 1) are looked at together, their loads in flight at once:
+// nearly every search ends there.
+template <int BPS, int S>
+__device__ uint32_t classic_target(const uint32_t *lat, const uint8_t *sites, const Geometry &g, uint32_t idx)
+{
+    const uint32_t zc = idx / g.XY, rem = idx - zc * g.XY, yc = rem / g.X, xc = rem - yc * g.X;
+    const uint32_t at[7] = {idx,
+                            xc > 0 ? idx - 1u : NO_SITE,
+                            yc > 0 ? idx - g.X : NO_SITE,
+                            zc > 0 ? idx - g.XY : NO_SITE,
+                            zc + 1u < g.Z ? idx + g.XY : NO_SITE,
+                            yc + 1u < g.Y ? idx + g.X : NO_SITE,
+                            xc + 1u < g.X ? idx + 1u : NO_SITE};
+    uint8_t type[7];
+    bool room[7];
+#pragma unroll
+    for (int j = 0; j < 7; j++) {
+        const uint32_t i = at[j] != NO_SITE ? at[j] : idx;
+        type[j] = sites[i];
+        room[j] = has_room<BPS, S>(lat, g.N, i);
+    }
+    const uint8_t tc = type[0];
+    uint32_t ok = 0;
+#pragma unroll
+    for (int j = 0; j < 7; j++) ok |= (at[j] != NO_SITE && type[j] == tc && room[j] ? 1u : 0u) << j;
+#pragma unroll
+    for (int j = 0; j < 7; j++)
+        if ((ok >> j) & 1u) return at[j];
+    for (uint32_t radius = 2; radius <= 4; radius++) {
+        const uint32_t mind = radius - 1u, maxd = radius;
+        const uint32_t min2 = mind * mind, max2 = maxd * maxd;
         const uint32_t x0 = xc >= maxd ? xc - maxd : 0, x1 = (xc + maxd < g.X) ? xc + maxd : g.X - 1;
         const uint32_t y0 = yc >= maxd ? yc - maxd : 0, y1 = (yc + maxd < g.Y) ? yc + maxd : g.Y - 1;
         const uint32_t z0 = zc >= maxd ? zc - maxd : 0, z1 = (zc + maxd < g.Z) ? zc + maxd : g.Z - 1;
         for (uint32_t x = x0; x <= x1; x++)
             for (uint32_t y = y0; y <= y1; y++)
                 for (uint32_t z = z0; z <= z1; z++) {
-                    const double dx = (double)x - xc, dy = (double)y - yc, dz = (double)z - zc;
-                    const double r2 = dx * dx + dy * dy + dz * dz;
-                    if (!(r2 <= max2 && (r2 > min2 || mind == maxd))) continue;
+                    const int32_t dx = (int32_t)(x - xc), dy = (int32_t)(y - yc), dz = (int32_t)(z - zc);
+                    const uint32_t r2 = (uint32_t)(dx * dx + dy * dy + dz * dz);
+                    if (r2 > max2 || r2 <= min2) continue;
                     const uint32_t j = x + y * g.X + z * g.XY;
-                    if (sites[j] == tc && occupancy_at<BPS, S>(lat, g.N, j) < (uint32_t)S)
-                        if (add_particle<BPS, S>(lat, g.N, j, p, pb)) return true;
+                    if (sites[j] == tc && has_room<BPS, S>(lat, g.N, j)) return j;
                 }
     }
-    return false;
+    return NO_SITE;
 }
 
 // Smallest power of two >= n (n >= 1).
@@ -108,7 +130,7 @@ __host__ __device__ __forceinline__ uint32_t pow2_at_least(uint32_t n)
 // counts of the lattice being taken, to which every particle put back is
 // added.
 template <int BPS, int S>
-__device__ void resolve_block_flat(uint32_t *lat, const uint8_t *sites, const Geometry &g, RunState *rs,
+__device__ __noinline__ void resolve_block_flat(uint32_t *lat, const uint8_t *sites, const Geometry &g, RunState *rs,
                                    OverflowEntry *list, uint32_t cap, OverflowEntry *sh, uint32_t tid,
                                    uint32_t nthreads, uint32_t *pb, unsigned long long *counts = nullptr)
 {
@@ -141,37 +163,98 @@ __device__ void resolve_block_flat(uint32_t *lat, const uint8_t *sites, const Ge
         }
     }
     __syncthreads();
-    // Bitonic sort by key.
-    for (uint32_t k = 2; k <= p2; k <<= 1) {
-        for (uint32_t j = k >> 1; j > 0; j >>= 1) {
-            for (uint32_t e = tid; e < p2; e += nthreads) {
-                const uint32_t o = e ^ j;
-                if (o > e) {
-                    const bool up = (e & k) == 0;
-                    const OverflowEntry a = sh[e], b = sh[o];
-                    if ((a.key > b.key) == up) {
-                        sh[e] = b;
-                        sh[o] = a;
+    if (n <= nthreads) {
+        // Few entries: each thread counts the keys below its entry's (keys
+        // are distinct) and moves it there.
+        OverflowEntry v = {0ull, 0u, 0u};
+        uint32_t rank = 0;
+        if (tid < n) {
+            v = sh[tid];
+            for (uint32_t e = 0; e < n; e++) rank += sh[e].key < v.key ? 1u : 0u;
+        }
+        __syncthreads();
+        if (tid < n) sh[rank] = v;
+        __syncthreads();
+    } else {
+        // Bitonic sort by key.
+        for (uint32_t k = 2; k <= p2; k <<= 1) {
+            for (uint32_t j = k >> 1; j > 0; j >>= 1) {
+                for (uint32_t e = tid; e < p2; e += nthreads) {
+                    const uint32_t o = e ^ j;
+                    if (o > e) {
+                        const bool up = (e & k) == 0;
+                        const OverflowEntry a = sh[e], b = sh[o];
+                        if ((a.key > b.key) == up) {
+                            sh[e] = b;
+                            sh[o] = a;
+                        }
                     }
                 }
+                __syncthreads();
             }
-            __syncthreads();
         }
     }
-    if (tid != 0) return;
-    rs->overflows += (unsigned long long)(n - carried);
+    if (tid == 0) rs->overflows += (unsigned long long)(n - carried);
     if (rs->mode == LMB_OVERFLOW_CLASSIC) {
-        for (uint32_t e = 0; e < n; e++) {
-            if (!reinsert_classic<BPS, S>(lat, sites, g, sh[e].site, sh[e].particle, pb)) {
-                rs->status = LMB_E_OVERFLOW_UNRESOLVED;
-                rs->failed_step = rs->step;
+        // One entry per thread, in queue order.  Every thread finds its
+        // entry's target from the lattice as it stands.  An insertion only
+        // ever takes room away, from its own target, so an entry's target is
+        // the one a search entry by entry finds as long as the target still
+        // has room after the entries before it with the same one; they fill
+        // its slots in order.  Up to the first entry for which it has none
+        // left (or which has no target at all) everything is inserted at
+        // once, and the rest search again.  (Entry by entry, each search and
+        // insertion a chain of L2 round trips with the whole device waiting,
+        // 107 entries of a 64^3 lattice took over 30 us of a timestep.)
+        __shared__ uint32_t s_first;
+        for (uint32_t base = 0; base < n;) {
+            const uint32_t cnt = n - base < nthreads ? n - base : nthreads;
+            const bool mine = tid < cnt;
+            OverflowEntry v = {0ull, 0u, 0u};
+            uint32_t target = NO_SITE, held = 0;
+            if (tid == 0) s_first = cnt;
+            if (mine) {
+                v = sh[base + tid];
+                target = classic_target<BPS, S>(lat, sites, g, v.site);
+                if (target != NO_SITE) {
+                    SiteWords<BPS, S> w;
+                    load_site_cg<BPS, S>(lat, g.N, target, w);
+                    held = (uint32_t)__popc(occupied_slots<BPS, S>(w));
+                }
+                sh[base + tid].key = target;  // the keys have served
+            }
+            __syncthreads();
+            uint32_t slot = held;
+            if (mine) {
+                for (uint32_t e = 0; e < tid; e++) slot += (uint32_t)sh[base + e].key == target ? 1u : 0u;
+                if (target == NO_SITE || slot >= (uint32_t)S) atomicMin(&s_first, tid);
+            }
+            __syncthreads();
+            const uint32_t take = s_first;
+            if (tid < take) {
+                if (BPS == 1)
+                    reinterpret_cast<uint8_t *>(lat + (size_t)(slot >> 2) * g.N + target)[slot & 3u] = (uint8_t)v.particle;
+                else
+                    lat[(size_t)slot * g.N + target] = v.particle;
+                cover_slot<BPS>(pb, target, slot);
+                if (counts) atomicAdd(counts + v.particle, 1ull);
+            }
+            const bool failed = take < cnt && (uint32_t)sh[base + take].key == NO_SITE;
+            __syncthreads();
+            if (failed) {  // the entries before it are in place
+                if (tid == 0) {
+                    rs->status = LMB_E_OVERFLOW_UNRESOLVED;
+                    rs->failed_step = rs->step;
+                }
                 return;
             }
-            if (counts) atomicAdd(counts + sh[e].particle, 1ull);
+            base += take;
         }
-        rs->ovf_count = 0;
-        rs->carried = 0;
-    } else {
+        if (tid == 0) {
+            rs->ovf_count = 0;
+            rs->carried = 0;
+        }
+    } else if (tid == 0) {
         // Relaxed (MpdRdmeSolver.cu:1677-1761): own site only; the rest stay
         // queued, in order, for the next timestep.
         uint32_t kept = 0;
@@ -188,7 +271,7 @@ __device__ void resolve_block_flat(uint32_t *lat, const uint8_t *sites, const Ge
         rs->carried = kept;
     }
     __threadfence();
-    set_step(rs, rs->seed, rs->step + 1);
+    if (tid == 0) set_step(rs, rs->seed, rs->step + 1);
 }
 
 template <int BPS, int S>

@@ -20,8 +20,9 @@
 // solve is given one at admission (in turn), and each stream advances its
 // oldest solve in every step, so that large solves finish in arrival order
 // per stream instead of all finishing late.  A large solve takes the
-// schedule that suits its particle density: the per-phase kernels for dense
-// lattices, the fused kernel for sparse ones.
+// lattice's own default, particle-list tiles planned for its density; where
+// those do not fit, the per-phase kernels for dense lattices and the dense
+// fused kernel for sparse ones.
 //
 // Host code only; it drives the device through the C ABI of lmb_capi.cu.
 #include <chrono>
@@ -303,7 +304,7 @@ static int admit(lmb_server *s)
         int rc = lmb_model_create(c, &d, a.req.X, a.req.Y, a.req.Z, &a.model);
         if (rc == LMB_OK) rc = lmb_lattice_create(c, a.req.X, a.req.Y, a.req.Z, s->slots, s->bps, &a.lat);
         if (rc == LMB_OK) rc = lmb_lattice_set_native(a.lat, a.req.particles.data(), a.req.sites.data());
-        if (rc == LMB_OK && a.solo) {
+        if (rc == LMB_OK && a.solo && !lmb::lattice_by_particle(a.lat)) {
             const double density = (double)count_particles(a.req.particles, s->bps) / (double)nsites;
             if (density >= DENSE_PARTICLES_PER_SITE) rc = lmb_lattice_set_schedule(a.lat, LMB_SCHEDULE_PHASES, 0, 0);
         }

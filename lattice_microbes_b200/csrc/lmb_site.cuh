@@ -374,15 +374,22 @@ __device__ __forceinline__ ReactBound react_bound(uint32_t t, const DevTables &m
     return ReactBound{tload(m.qp0 + t), tload(m.qpmax + t), tload(m.qpmax + m.nst + t)};
 }
 
-__device__ __forceinline__ bool reaction_may_fire(uint32_t n, const ReactBound &b, float r0)
+// The bound itself; it does not fall with n (n >= 1: every step is monotone
+// and rounded upwards).
+__device__ __forceinline__ float reaction_bound(uint32_t n, const ReactBound &b)
 {
-    if (n == 0 && b.a0 == 0.0f) return false;
     const float nf = (float)n;
     const float pairs = __fmul_rn(nf, __fmul_rn(__fsub_rn(nf, 1.0f), 0.5f));
     float u = __fadd_ru(b.a0, __fmul_ru(nf, b.q1));
     u = __fadd_ru(u, __fmul_ru(pairs, b.q2));
     u = __fmul_ru(u, 1.0001f);
-    return !(r0 > __fadd_ru(__fmul_ru(u, 1.00000095367431640625f), 8.67361738e-19f));
+    return __fadd_ru(__fmul_ru(u, 1.00000095367431640625f), 8.67361738e-19f);
+}
+
+__device__ __forceinline__ bool reaction_may_fire(uint32_t n, const ReactBound &b, float r0)
+{
+    if (n == 0 && b.a0 == 0.0f) return false;
+    return !(r0 > reaction_bound(n, b));
 }
 
 __device__ __forceinline__ bool reaction_may_fire(uint32_t n, float a0, uint32_t t, float r0, const DevTables &m)
@@ -395,7 +402,9 @@ __device__ __forceinline__ bool reaction_may_fire(uint32_t n, float a0, uint32_t
 // one reaction; returns true when the site changed (s updated in place).
 // CAP > 0: the reaction's candidates are sorted in a list of CAP registers
 // (nothing in local memory; for kernels whose registers are scarce and whose
-// models have few candidates per site); CAP == 0: in a 64-entry array.
+// models have few candidates per site); CAP == 0: in a bitmap over the model's
+// reactions (a 64-entry array past 4096 of them); CAP < 0: models of up to 32
+// reactions, the bitmap in one register.
 template <int BPS, int S, int CAP>
 __device__ __forceinline__ bool react_site(SiteWords<BPS, S> &s, uint32_t t, uint32_t gi, unsigned long long th,
                                            const DevTables &m, RunState *rs, OverflowEntry *list, uint32_t cap)
@@ -453,12 +462,12 @@ __device__ __forceinline__ bool react_site(SiteWords<BPS, S> &s, uint32_t t, uin
             rp = __fsub_rn(rp, prop);
         }
     };
-    constexpr int LEN = CAP > 0 ? CAP : 64;
+    constexpr int LEN = CAP > 0 ? CAP : (CAP < 0 ? 1 : 64);
     // CAP == 0, models of up to BMW * 32 reactions: the candidates are the
     // set bits of a bitmap indexed by reaction, which keeps them sorted and
     // drops repeats whatever their number (a full site of one species, say).
-    constexpr uint32_t BMW = CAP > 0 ? 1 : 128;
-    const bool bitmap = CAP == 0 && m.nr <= BMW * 32;
+    constexpr uint32_t BMW = CAP != 0 ? 1 : 128;
+    const bool bitmap = CAP < 0 || (CAP == 0 && m.nr <= BMW * 32);
     // Only its first nbw words are used, each cleared below before any bit
     // is set (the compiler cannot see that the two conditions agree).
 #pragma nv_diag_suppress 549
@@ -490,7 +499,7 @@ __device__ __forceinline__ bool react_site(SiteWords<BPS, S> &s, uint32_t t, uin
             }
             nc++;
         } else if (bitmap) {
-            bm[v >> 5] |= 1u << (v & 31u);
+            bm[CAP < 0 ? 0u : v >> 5] |= 1u << (v & 31u);
         } else {
             if (nc < LEN) cand[nc++] = v;
             else all = true;
@@ -500,9 +509,9 @@ __device__ __forceinline__ bool react_site(SiteWords<BPS, S> &s, uint32_t t, uin
 #pragma unroll
         for (int j = 0; j < LEN; j++) cand[j] = 0xFFFFFFFFu;
     }
-    const uint32_t nbw = (m.nr + 31u) / 32u;
+    const uint32_t nbw = CAP < 0 ? 1u : (m.nr + 31u) / 32u;
     if (bitmap)
-        for (uint32_t w = 0; w < nbw; w++) bm[w] = 0u;
+        for (uint32_t w = 0; w < nbw; w++) bm[CAP < 0 ? 0u : w] = 0u;
     {
         const uint32_t z0 = tload(m.rx_off), z1 = tload(m.rx_off + 1);
         for (uint32_t e = z0; e < z1 && !all; e++) insert(tload(m.rx_list + e));
@@ -558,7 +567,7 @@ __device__ __forceinline__ bool react_site(SiteWords<BPS, S> &s, uint32_t t, uin
             nb = 0;
         };
         for (uint32_t w = 0; w < nbw; w++) {
-            uint32_t bits = bm[w];
+            uint32_t bits = bm[CAP < 0 ? 0u : w];
             while (bits) {
                 const uint32_t k = __ffs(bits) - 1;
                 bits &= bits - 1;

@@ -106,3 +106,29 @@ def test_species_past_a_list_entry(ctx, X, slots):
         big.S[ids[s + 1] - 1], big.D[ids[s + 1] - 1] = spec.S[s], spec.D[s]
         big.DF[:, :, ids[s + 1] - 1] = spec.DF[:, :, s]
     _run(ctx, big, 3, (4, 4) if X == 128 else (2, 2))
+
+
+@pytest.mark.parametrize("slots,bps,density", [(8, 1, 2.6), (8, 1, 4.2), (16, 1, 9.6), (4, 4, 1.7), (16, 4, 9.6)])
+@pytest.mark.parametrize("schedule", ["fused", "phases"])
+def test_many_overflows_in_a_timestep(ctx, slots, bps, density, schedule):
+    """From tens to more overflows than a block has threads in one timestep,
+    many of them into the same sites: the insertions made together equal the
+    oracle's, made one after another."""
+    from lattice_microbes_b200 import _lib as L
+    from lattice_microbes_b200.solver import Lattice, Model
+    spec = configs.random_problem(61, X=64, Y=16, Z=16, slots=slots, bytes_per_slot=bps, density=density, nst=2,
+                                  zeroth=False)
+    t = oracle_tables(spec)
+    model = Model.from_tables(ctx, t)
+    lat = Lattice(ctx, spec.X, spec.Y, spec.Z, slots, bps)
+    lat.set_schedule(L.LMB_SCHEDULE_FUSED if schedule == "fused" else L.LMB_SCHEDULE_PHASES)
+    lat.set_native(spec.lattice, spec.sites)
+    rc, st = lat.run(model, 5, 0, 4, check=False)
+    ref, rc_ref, st_ref = oracle_run(t, spec.lattice, spec.sites, 5, 0, 4)
+    assert rc == rc_ref
+    assert st_ref.overflows > 40
+    assert st.overflows == st_ref.overflows
+    out, _ = lat.get_native()
+    assert np.array_equal(out, ref)
+    lat.close()
+    model.close()
