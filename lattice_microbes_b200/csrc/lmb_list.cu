@@ -231,21 +231,34 @@ __device__ __forceinline__ void list_rows(const uint32_t *__restrict__ src, cons
     constexpr uint32_t W = SiteWords<BPS, S>::W;
     constexpr uint32_t EARLY = W < 2 ? W : 2;
     const uint32_t nit = rows * q;
-    for (uint32_t i0 = 0; i0 < nit; i0 += NT) {
-        const uint32_t i = i0 + threadIdx.x;
-        uint32_t v[EARLY][V], l0 = 0, g0 = 0, npl = 0;
+    // The next item's loads are in flight while this one is listed: a region
+    // is several iterations long, each a round trip to L2 otherwise.
+    uint32_t v[EARLY][V], w[EARLY][V], l0 = 0, g0 = 0, npl = 0, l1 = 0, g1 = 0, npl1 = 0;
+    auto fetch = [&](uint32_t i) {
+        l1 = g1 = npl1 = 0;
 #pragma unroll
         for (uint32_t k = 0; k < EARLY; k++)
 #pragma unroll
-            for (int j = 0; j < V; j++) v[k][j] = 0u;
+            for (int j = 0; j < V; j++) w[k][j] = 0u;
         if (i < nit) {
             const uint32_t r = fast_div(i, mq), c = i - r * q;
-            l0 = r * X + c * V;
-            g0 = rowbase[r] + c * V;
+            l1 = r * X + c * V;
+            g1 = rowbase[r] + c * V;
 #pragma unroll
-            for (uint32_t k = 0; k < EARLY; k++) load_sites<V>(src + (size_t)k * N + g0, v[k]);
-            if (W > EARLY) npl = pb ? min(pb[g0 >> PB_SHIFT], W) : W;
+            for (uint32_t k = 0; k < EARLY; k++) load_sites<V>(src + (size_t)k * N + g1, w[k]);
+            if (W > EARLY) npl1 = pb ? min(pb[g1 >> PB_SHIFT], W) : W;
         }
+    };
+    fetch(threadIdx.x);
+    for (uint32_t i0 = 0; i0 < nit; i0 += NT) {
+#pragma unroll
+        for (uint32_t k = 0; k < EARLY; k++)
+#pragma unroll
+            for (int j = 0; j < V; j++) v[k][j] = w[k][j];
+        l0 = l1;
+        g0 = g1;
+        npl = npl1;
+        if (i0 + NT < nit) fetch(i0 + NT + threadIdx.x);
         uint32_t n = 0;
         bool held[EARLY];
 #pragma unroll
@@ -270,11 +283,11 @@ __device__ __forceinline__ void list_rows(const uint32_t *__restrict__ src, cons
         if constexpr (W > EARLY) {
             const uint32_t most = __reduce_max_sync(0xffffffffu, npl);
             for (uint32_t k = EARLY; k < most; k++) {
-                uint32_t w[V];
+                uint32_t u[V];
 #pragma unroll
-                for (int j = 0; j < V; j++) w[j] = 0u;
-                if (k < npl) load_sites<V>(src + (size_t)k * N + g0, w);
-                list_plane<BPS, V>(w, l0, k, list, C, count);
+                for (int j = 0; j < V; j++) u[j] = 0u;
+                if (k < npl) load_sites<V>(src + (size_t)k * N + g0, u);
+                list_plane<BPS, V>(u, l0, k, list, C, count);
             }
         }
     }
@@ -876,18 +889,22 @@ __global__ void __launch_bounds__(NT, MINB) list_step_kernel(const uint32_t *__r
                           blockIdx.x, gridDim.x);
 }
 
-// A batch of lattices advanced together, as fused_batch_kernel does it.
+// A batch of lattices advanced together, as fused_batch_kernel does it.  The
+// threads look for the block's job side by side (a binary search is a chain of
+// round trips), and the job is worked from a copy in shared memory.
 template <int BPS, int S, int NT, int MINB>
 __global__ void __launch_bounds__(NT, MINB) list_batch_kernel(const FusedJob *__restrict__ jobs, uint32_t njobs,
                                                              uint32_t parity, uint32_t smem_bytes)
 {
-    uint32_t lo = 0, hi = njobs;
-    while (hi - lo > 1) {
-        const uint32_t mid = (lo + hi) / 2;
-        if (jobs[mid].tile_begin <= blockIdx.x) lo = mid;
-        else hi = mid;
-    }
-    const FusedJob &j = jobs[lo];
+    __shared__ uint32_t s_job;
+    __shared__ __align__(16) uint32_t s_copy[(sizeof(FusedJob) + 3) / 4];
+    for (uint32_t j = threadIdx.x; j < njobs; j += NT)
+        if (jobs[j].tile_begin <= blockIdx.x && (j + 1u == njobs || jobs[j + 1u].tile_begin > blockIdx.x)) s_job = j;
+    __syncthreads();
+    const uint32_t *from = reinterpret_cast<const uint32_t *>(jobs + s_job);
+    for (uint32_t w = threadIdx.x; w < sizeof(FusedJob) / 4u; w += NT) s_copy[w] = from[w];
+    __syncthreads();
+    const FusedJob &j = *reinterpret_cast<const FusedJob *>(s_copy);
     const uint32_t c = j.cur0 ^ parity;
     list_tile<BPS, S, NT>(j.buf[c], j.buf[c ^ 1], j.sites, j.g, j.m, j.rs, j.list, j.cap, j.ts, j.with_reaction,
                           nullptr, nullptr, smem_bytes, blockIdx.x - j.tile_begin, j.ts.tiles_y * j.ts.tiles_z);
