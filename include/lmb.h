@@ -41,7 +41,9 @@ extern "C" {
 #define LMB_OVERFLOW_RELAXED 1
 
 /* Timestep schedules.  FUSED runs the x, y, z sweeps and the reaction of a
- * tile of Ty x Tz full x-rows in shared memory, one launch per timestep;
+ * tile of Ty x Tz full x-rows in shared memory, one launch per timestep (the
+ * tile's particles in a list, whose length follows the lattice's density;
+ * with Ty = Tz = 0 the tile does too);
  * PHASES launches one kernel per sweep, the reaction and the overflow pass
  * (the reference's schedule, MpdRdmeSolver.cu:1011-1090); CLUSTER, for small
  * lattices, holds the whole lattice in the shared memory of one thread-block
@@ -190,8 +192,8 @@ int lmb_lattice_get_row_major(lmb_lattice *lattice, void *particles, uint8_t *si
 int lmb_lattice_set_schedule(lmb_lattice *lattice, int schedule, uint32_t Ty, uint32_t Tz);
 int lmb_lattice_get_schedule(lmb_lattice *lattice, int *schedule, uint32_t *Ty, uint32_t *Tz);
 /* Autotuner: times the per-phase schedule, the cluster-resident one where it
- * fits and every fused tile shape that fits for `timesteps` on a saved copy
- * of the lattice state, restores the state and keeps the fastest.  The
+ * fits and the fused tile shapes with the best estimates for `timesteps` on a
+ * saved copy of the lattice state, restores the state and keeps the fastest.  The
  * grid-resident schedule is chosen only by lmb_lattice_set_schedule: its
  * cooperative launch does not overlap other lattices' runs on other streams,
  * which fused launches do. */
@@ -256,8 +258,8 @@ int lmb_run_native_async(lmb_lattice *lattice, const lmb_model *model, uint32_t 
  * the run (recordSpeciesCounts, MpdRdmeSolver.cu:933-942, with
  * ByteLattice::getParticleCounts, ByteLattice.cpp:495-520) inside the run's
  * own work: on the fused schedule the last timestep's kernel adds the
- * particles of the sites each block stores into per-block histograms, one
- * atomic per species, and the overflow resolution adds those it puts back;
+ * particles each block stores into per-block histograms, one atomic per
+ * species, and the overflow resolution adds those it puts back;
  * on the per-phase schedule one pass after the last timestep reads only the
  * word planes below each segment's plane bound.  The totals come back with
  * the run state: lmb_run_counts_wait returns them, counts[0..number_species]
@@ -331,8 +333,9 @@ int lmb_batch_destroy(lmb_batch *batch);
  * retires the solves that are done.  Solves of at least 131,072 sites
  * (which fill the device alone) run their chunks on their own instead, on
  * two streams beside the small solves' batch (each stream one solve at a
- * time, in arrival order), with the per-phase schedule when they hold 0.05
- * particles per site or more.  A solve's result is lmb_run's result for it
+ * time, in arrival order), on fused tiles planned for their density (the
+ * per-phase schedule for layouts without particle-list tiles that hold 0.05
+ * particles per site or more).  A solve's result is lmb_run's result for it
  * alone, bit for bit.  Replaces the reference's one-solver-per-thread
  * replicate runner (core/ReplicateRunner.cpp:84-166) for many independent
  * solves on one device. */
