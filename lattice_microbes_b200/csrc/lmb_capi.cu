@@ -93,11 +93,13 @@ struct lmb_lattice {
     // lattice.
     float density, plan_density;
     bool auto_plan;
-    // Captured timestep graphs, one per starting buffer parity.
+    // Captured timestep graphs, one per starting buffer parity, with what the
+    // captured launches were given.  The table set is compared whole: the
+    // kernels take it by value, and a rate change rewrites the tables in
+    // place but not the set a captured launch holds.
     struct Graph {
         cudaGraphExec_t exec;
-        const void *model;
-        const void *tables;
+        DevTables tables;
         int schedule;
         uint32_t Ty, Tz, list_smem;
         bool reaction;
@@ -401,6 +403,7 @@ static lmb_model *new_model(lmb_ctx *c, uint32_t ns, uint32_t nst, uint32_t nr)
     m->tau = 0;
     m->dev_block = nullptr;
     m->dev_bytes = 0;
+    memset(&m->dev, 0, sizeof(m->dev));  // the padding too: table sets are compared as bytes
     m->dirty = true;
     m->T.assign((size_t)nst * nst * ns, 0.0f);
     m->qp0.assign(nst, 0.0f);
@@ -990,13 +993,13 @@ static cudaError_t reset_plane_bounds(lmb_lattice *l, const lmb_model *m, cudaSt
 }
 
 // Captures GRAPH_STEPS timesteps starting at the current buffer parity, or
-// keeps the graph captured before for the same model storage and schedule.
+// keeps the graph captured before for the same table set and schedule.
 // Every kernel reads the step index from the run state, so one graph serves
 // any run.
 static int ensure_graph(lmb_lattice *l, lmb_model *m)
 {
     lmb_lattice::Graph &gr = l->graph[l->cur];
-    const bool same = gr.exec && gr.model == m && gr.tables == m->dev_block && gr.schedule == l->schedule &&
+    const bool same = gr.exec && memcmp(&gr.tables, &m->dev, sizeof(DevTables)) == 0 && gr.schedule == l->schedule &&
                       gr.Ty == l->tile.Ty && gr.Tz == l->tile.Tz && gr.list_smem == l->tile.list_smem &&
                       gr.reaction == (m->nr > 0);
     if (same) return LMB_OK;
@@ -1028,8 +1031,7 @@ static int ensure_graph(lmb_lattice *l, lmb_model *m)
         gr.exec = nullptr;
         return cuda_status(e);
     }
-    gr.model = m;
-    gr.tables = m->dev_block;
+    memcpy(&gr.tables, &m->dev, sizeof(DevTables));
     gr.schedule = l->schedule;
     gr.Ty = l->tile.Ty;
     gr.Tz = l->tile.Tz;

@@ -132,3 +132,39 @@ def test_many_overflows_in_a_timestep(ctx, slots, bps, density, schedule):
     assert np.array_equal(out, ref)
     lat.close()
     model.close()
+
+
+@pytest.mark.parametrize("slots,bps", [(8, 1), (16, 4)])
+def test_zeroth_order_rate_switched_on_between_runs(ctx, slots, bps):
+    """A source whose rate is 0 for 64 timesteps (a captured graph) and
+    positive for the next 64: empty sites produce from then on, however the
+    run is cut."""
+    from lattice_microbes_b200.solver import Lattice, Model
+    spec = configs.random_problem(71, X=32, Y=16, Z=16, slots=slots, bytes_per_slot=bps, density=0.01)
+    src = [j for j in range(spec.nr) if spec.rtype[j] == configs.ZEROTH]
+    spec.RL[src] = 1
+    on = spec.K.copy()
+    on[src] *= 0.1
+    spec.K[src] = 0.0
+    off = oracle_tables(spec)
+    spec.K = on
+    lit = oracle_tables(spec)
+    assert not off.qp0.any() and lit.qp0.all()
+    mid, rc, _ = oracle_run(off, spec.lattice, spec.sites, 13, 0, 64)
+    ref, rc2, st_ref = oracle_run(lit, mid, spec.sites, 13, 64, 64)
+    assert rc == rc2 == 0 and st_ref.reactions > 1000
+    for piece in (64, 16):
+        spec.K = on.copy()
+        spec.K[src] = 0.0
+        model = Model.from_spec(ctx, spec)
+        lat = Lattice(ctx, spec.X, spec.Y, spec.Z, slots, bps)
+        lat.set_native(spec.lattice, spec.sites)
+        for t in range(0, 128, piece):
+            if t == 64:
+                for j in src:
+                    model.set_reaction_rate(j, float(on[j]))
+            lat.run(model, 13, t, piece)
+        out, _ = lat.get_native()
+        assert np.array_equal(out, ref), piece
+        lat.close()
+        model.close()
