@@ -127,8 +127,8 @@ __host__ __device__ __forceinline__ uint32_t pow2_at_least(uint32_t n)
 // `nthreads`); `sh` holds pow2_at_least(cap) entries.  On success the step
 // counter advances.  pb: the lattice's plane bounds, raised for every slot
 // filled here (null when it keeps none).  counts (when not null): species
-// counts of the lattice being taken, to which every particle put back is
-// added.
+// counts 0 .. rs->count_ns of the lattice being taken, to which every particle
+// of those species put back is added.
 template <int BPS, int S>
 __device__ __noinline__ void resolve_block_flat(uint32_t *lat, const uint8_t *sites, const Geometry &g, RunState *rs,
                                    OverflowEntry *list, uint32_t cap, OverflowEntry *sh, uint32_t tid,
@@ -237,7 +237,7 @@ __device__ __noinline__ void resolve_block_flat(uint32_t *lat, const uint8_t *si
                 else
                     lat[(size_t)slot * g.N + target] = v.particle;
                 cover_slot<BPS>(pb, target, slot);
-                if (counts) atomicAdd(counts + v.particle, 1ull);
+                if (counts && v.particle <= rs->count_ns) atomicAdd(counts + v.particle, 1ull);
             }
             const bool failed = take < cnt && (uint32_t)sh[base + take].key == NO_SITE;
             __syncthreads();
@@ -263,7 +263,7 @@ __device__ __noinline__ void resolve_block_flat(uint32_t *lat, const uint8_t *si
                 OverflowEntry o = sh[e];
                 o.key = (unsigned long long)kept;  // phase 0, list order
                 list[kept++] = o;
-            } else if (counts) {
+            } else if (counts && sh[e].particle <= rs->count_ns) {
                 atomicAdd(counts + sh[e].particle, 1ull);
             }
         }

@@ -134,6 +134,26 @@ def test_many_overflows_in_a_timestep(ctx, slots, bps, density, schedule):
     model.close()
 
 
+@pytest.mark.parametrize("mode", [0, 1])
+@pytest.mark.parametrize("counted", [1, 3])
+def test_counts_of_fewer_species_than_overflow(ctx, counted, mode):
+    """Species totals asked for up to a species below those the overflow
+    resolution puts back in the counted timestep."""
+    from lattice_microbes_b200.solver import Lattice, Model
+    spec = configs.random_problem(61, X=64, Y=16, Z=16, slots=8, bytes_per_slot=1, density=2.6, nst=2, zeroth=False)
+    t = oracle_tables(spec)
+    model = Model.from_tables(ctx, t)
+    lat = Lattice(ctx, spec.X, spec.Y, spec.Z, 8, 1)
+    lat.set_native(spec.lattice, spec.sites)
+    ref, rc_ref, st_ref = oracle_run(t, spec.lattice, spec.sites, 5, 0, 1, mode)
+    assert rc_ref == 0 and st_ref.overflows > 40
+    rc, st, counts = lat.run_counts(model, 5, 0, 1, counted, mode)
+    assert st.overflows == st_ref.overflows
+    assert np.array_equal(counts, oracle_counts(t, ref)[: counted + 1])
+    lat.close()
+    model.close()
+
+
 @pytest.mark.parametrize("slots,bps", [(8, 1), (16, 4)])
 def test_zeroth_order_rate_switched_on_between_runs(ctx, slots, bps):
     """A source whose rate is 0 for 64 timesteps (a captured graph) and
