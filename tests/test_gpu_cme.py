@@ -157,3 +157,40 @@ def test_compact_kernel_equals_generic(ctx, model):
     assert fin_g == fin_a == 3000
     assert ev_g == ev_a and ev_g > 3000
     assert np.array_equal(gen, auto)
+
+
+@pytest.mark.parametrize("ns,nr", [(1, 1), (1, 3), (3, 3), (2, 4), (4, 4), (3, 5), (2, 6), (4, 6), (1, 7), (4, 7),
+                                   (2, 8), (4, 8)])
+@pytest.mark.parametrize("zeroth", [0, 1, 2])
+def test_linear_kernel_equals_generic(ctx, ns, nr, zeroth):
+    """Linear models over the species and reactions the linear kernel takes
+    (its forms hold up to 4, 6 and 8 reactions; fewer are padded), with no,
+    one and two sources, the reactions in mixed order, changes up to +7 and
+    -8: trajectories, records and event counts as the generic kernel gives
+    them, also in segments and with records between events."""
+    from lattice_microbes_b200 import _lib as L
+    rng = np.random.default_rng(100 * ns + 10 * nr + zeroth)
+    first = max(1, nr - zeroth)
+    rtype = np.array([1] * first + [0] * (nr - first), np.uint32)
+    rng.shuffle(rtype)
+    S = np.zeros((ns, nr), np.int32)
+    D = np.zeros((ns, nr), np.uint32)
+    K = np.zeros(nr)
+    for r in range(nr):
+        if rtype[r] == 0:
+            S[rng.integers(ns), r] = rng.integers(1, 8)
+            K[r] = rng.uniform(0.2, 1.0)
+        else:
+            # Mostly decays and conversions, so that counts stay finite.
+            a = rng.integers(ns)
+            D[a, r] = 1
+            S[a, r] -= 1 if rng.random() < 0.8 else 8
+            if rng.random() < 0.5:
+                S[rng.integers(ns), r] += 1
+            K[r] = rng.uniform(0.05, 0.4)
+    spec = configs.CMESpec("linear", ns, rtype, K, S, D, rng.integers(8, 40, ns).astype(np.uint32), 20.0, 0.25)
+    gen, ev_g, fin_g = _ensemble_with_kernel(ctx, spec, 1000, 5, L.LMB_CME_KERNEL_GENERIC)
+    auto, ev_a, fin_a = _ensemble_with_kernel(ctx, spec, 1000, 5, L.LMB_CME_KERNEL_AUTO, segments=3)
+    assert fin_g == fin_a == 1000
+    assert ev_g == ev_a > 1000
+    assert np.array_equal(gen, auto)
