@@ -490,7 +490,7 @@ __global__ void __launch_bounds__(CME_LINEAR_THREADS) cme_linear_kernel(const Cm
 }
 
 // [entry][species][replicate] -> [replicate][entry][species] for replicates
-// first .. first + count - 1: a transposition of rows = entries x species rows
+// first .. first + count - 1: a transposition of `rows` rows (entry, species)
 // through 32 x 32 tiles, `across` tiles along the replicates.
 __global__ void __launch_bounds__(256) cme_collect_kernel(const int32_t *__restrict__ planar,
                                                           uint32_t *__restrict__ counts, uint32_t rows, uint32_t reps,
@@ -549,7 +549,7 @@ struct lmb_cme {
     int32_t *init_dev;
     uint32_t init_per_replicate;
     int32_t *out;
-    uint32_t *collected;  // lmb_cme_get_counts: a piece of the records in its order
+    uint32_t *collected;  // lmb_cme_get_counts: a piece of the records in its order, at most CME_COLLECT_BYTES
     size_t collected_len;
     size_t out_entries;
     uint32_t entries;
@@ -863,10 +863,14 @@ extern "C" int lmb_cme_get_counts(lmb_cme *c, uint32_t *counts)
     if (!c || !counts) return LMB_E_ARG;
     if (!c->begun) return LMB_E_STATE;
     CKC(cudaSetDevice(c->ctx->device));
-    const uint32_t rows = c->entries * c->ns;
-    // The records change order on the device, in pieces of a bounded buffer.
-    uint32_t piece = (uint32_t)std::min<size_t>(c->reps, std::max<size_t>(32, CME_COLLECT_BYTES / 4 / rows / 32 * 32));
-    const size_t need = (size_t)piece * rows;
+    const size_t rows = (size_t)c->entries * c->ns;
+    // The records change order on the device, in pieces of at most
+    // CME_COLLECT_BYTES: whole replicates where 32 of them fit, parts of the
+    // rows of 32 replicates where not.
+    const size_t most = CME_COLLECT_BYTES / 4;
+    const uint32_t piece = (uint32_t)std::min<size_t>(c->reps, std::max<size_t>(32, most / rows / 32 * 32));
+    const size_t down = std::min(rows, most / piece);
+    const size_t need = piece * down;
     if (c->collected_len < need) {
         if (c->collected) cudaFree(c->collected);
         c->collected = nullptr;
@@ -876,12 +880,21 @@ extern "C" int lmb_cme_get_counts(lmb_cme *c, uint32_t *counts)
     }
     for (uint32_t first = 0; first < c->reps; first += piece) {
         const uint32_t count = std::min(piece, c->reps - first), across = (count + 31) / 32;
-        cme_collect_kernel<<<across * ((rows + 31) / 32), 256, 0, c->ctx->stream>>>(c->out, c->collected, rows,
-                                                                                  c->reps, first, count, across);
-        count_launch();
-        CKC(cudaGetLastError());
-        CKC(cudaMemcpyAsync(counts + (size_t)first * rows, c->collected, (size_t)count * rows * 4,
-                            cudaMemcpyDeviceToHost, c->ctx->stream));
+        for (size_t r0 = 0; r0 < rows; r0 += down) {
+            const uint32_t len = (uint32_t)std::min(down, rows - r0);
+            cme_collect_kernel<<<across * ((len + 31) / 32), 256, 0, c->ctx->stream>>>(
+                c->out + r0 * c->reps, c->collected, len, c->reps, first, count, across);
+            count_launch();
+            CKC(cudaGetLastError());
+            if (len == rows) {
+                CKC(cudaMemcpyAsync(counts + first * rows, c->collected, count * rows * 4, cudaMemcpyDeviceToHost,
+                                    c->ctx->stream));
+            } else {
+                for (uint32_t r = 0; r < count; r++)
+                    CKC(cudaMemcpyAsync(counts + (first + r) * rows + r0, c->collected + (size_t)r * len,
+                                        (size_t)len * 4, cudaMemcpyDeviceToHost, c->ctx->stream));
+            }
+        }
     }
     CKC(cudaStreamSynchronize(c->ctx->stream));
     return LMB_OK;

@@ -194,3 +194,29 @@ def test_linear_kernel_equals_generic(ctx, ns, nr, zeroth):
     assert fin_g == fin_a == 1000
     assert ev_g == ev_a > 1000
     assert np.array_equal(gen, auto)
+
+
+@pytest.mark.parametrize("reps,t_end,dt", [(40, 15.0, 1e-4), (3, 15.0, 1e-4), (50007, 4.0, 0.04)])
+def test_records_collected_in_pieces(ctx, reps, t_end, dt):
+    """Records past the 64 MB that change order at a time: parts of the rows
+    of 32 replicates (and of the 8 left over), a few replicates' rows at
+    once, and whole replicates with a remainder that 32 does not divide;
+    each equals the records on the device, transposed."""
+    import ctypes as C
+    import torch
+    from lattice_microbes_b200 import _lib as L
+    from lattice_microbes_b200.solver import CMEEnsemble
+    spec = configs.two_state_gene(max_time=t_end, write_interval=dt)
+    ens = CMEEnsemble(ctx, spec, reps)
+    ens.run(3, t_end, dt)
+    shape = (ens.entries(), 4, reps)
+    assert reps < 32 or np.prod(shape) * 4 > 64 << 20
+    p = L.vp()
+    L.check(L.lib().lmb_cme_device_counts(ens.handle, C.byref(p)))
+
+    class Records:
+        __cuda_array_interface__ = dict(shape=shape, typestr="<i4", data=(p.value, False), version=2)
+
+    planar = torch.as_tensor(Records(), device="cuda").cpu().numpy()
+    assert np.array_equal(ens.counts(), planar.transpose(2, 0, 1).astype(np.uint32))
+    ens.close()
