@@ -822,11 +822,12 @@ extern "C" int lmb_lattice_set_row_major(lmb_lattice *l, const void *particles, 
                                   c->stream));
     CK(cudaMemcpyAsync(l->rs_host, l->rs, sizeof(RunState), cudaMemcpyDeviceToHost, c->stream));
     CK(cudaStreamSynchronize(c->stream));
-    // RDMESolver.cpp:160-185 rejects invalid species ids and site types.
+    // RDMESolver.cpp:160-185 rejects invalid species ids and site types.  The
+    // lattice holds them all the same: a run has to look at it again.
+    l->validated = false;
     if (l->rs_host->max_species > number_species || l->rs_host->max_site_type >= number_site_types) {
         return LMB_E_ARG;
     }
-    l->validated = false;
     return LMB_OK;
 }
 

@@ -86,3 +86,34 @@ def test_rejected_sizes_and_layouts(ctx):
     assert lib.lmb_lattice_create(ctx.handle, 8, 8, 8, 12, 1, C.byref(h)) == L.LMB_E_UNSUPPORTED
     assert lib.lmb_lattice_create(ctx.handle, 8, 8, 8, 32, 4, C.byref(h)) == L.LMB_E_UNSUPPORTED
     assert lib.lmb_lattice_create(ctx.handle, 8, 8, 8, 8, 2, C.byref(h)) == L.LMB_E_UNSUPPORTED
+
+
+@pytest.mark.parametrize("what", ["species", "site type"])
+@pytest.mark.parametrize("slots,bps", [(8, 1), (16, 4)])
+def test_refused_row_major_contents_do_not_run(ctx, slots, bps, what):
+    """Row-major contents refused for a species id or site type out of range
+    are in the lattice all the same; a run on it is refused until valid
+    contents are set."""
+    from lattice_microbes_b200 import _lib as L
+    from lattice_microbes_b200.solver import Lattice, Model
+    spec = configs.random_problem(34, X=32, Y=8, Z=8, slots=slots, bytes_per_slot=bps, density=0.5)
+    t = oracle_tables(spec)
+    model = Model.from_tables(ctx, t)
+    lat = Lattice(ctx, spec.X, spec.Y, spec.Z, slots, bps)
+    lat.set_native(spec.lattice, spec.sites)
+    assert lat.run(model, 3, 0, 2)[0] == 0
+    particles, sites = lat.get_row_major()
+    bad_p, bad_s = particles.copy(), sites.copy()
+    if what == "species":
+        bad_p[3, 2, 1, 0] = spec.ns + 1
+    else:
+        bad_s[3, 2, 1] = spec.nst
+    with pytest.raises(L.LmbError):
+        lat.set_row_major(bad_p, bad_s, spec.ns, spec.nst)
+    assert lat.run(model, 3, 2, 2, check=False)[0] == L.LMB_E_ARG
+    lat.set_row_major(particles, sites, spec.ns, spec.nst)
+    assert lat.run(model, 3, 2, 2)[0] == 0
+    ref, _, _ = oracle_run(t, spec.lattice, spec.sites, 3, 0, 4)
+    assert np.array_equal(lat.get_native()[0], ref)
+    lat.close()
+    model.close()
