@@ -85,6 +85,7 @@ struct lmb_lattice {
     uint32_t pending_count_ns;
     bool validated;
     uint32_t max_species, max_site_type;
+    uint32_t run_species;  // most species of a model with reactions run since the check
     // Schedule: fused tile kernel (one launch per timestep) or per-phase kernels.
     int schedule;
     TileShape tile;
@@ -1042,9 +1043,11 @@ static int ensure_graph(lmb_lattice *l, lmb_model *m)
     return LMB_OK;
 }
 
+// Checks the contents against the model: new contents, and contents a model of
+// more species may have added to (its reactions make species this one lacks).
 static int validate_for_model(lmb_lattice *l, const lmb_model *m)
 {
-    if (!l->validated) {
+    if (!l->validated || l->run_species > m->ns) {
         lmb_ctx *c = l->ctx;
         CK(cudaMemcpyAsync(l->rs_host, l->rs, sizeof(RunState), cudaMemcpyDeviceToHost, c->stream));
         CK(cudaStreamSynchronize(c->stream));
@@ -1059,11 +1062,13 @@ static int validate_for_model(lmb_lattice *l, const lmb_model *m)
         l->max_site_type = l->rs_host->max_site_type;
         l->density = (float)((double)l->rs_host->occupied / l->g.N);
         l->validated = true;
+        l->run_species = 0;
     }
     // Species ids index the qp tables unchecked on the device
     // (MpdRdmeSolver.cu:1617-1636), as the reference assumes after
     // RDMESolver::setLatticeData validated them.
     if (l->max_species > m->ns || l->max_site_type >= m->nst) return LMB_E_ARG;
+    if (m->nr > 0) l->run_species = std::max(l->run_species, m->ns);
     return LMB_OK;
 }
 
@@ -1090,6 +1095,7 @@ static int run_async(lmb_lattice *l, const lmb_model *mc, uint32_t seed, uint32_
     }
     int rc = device_check ? LMB_OK : validate_for_model(l, m);
     if (rc) return rc;
+    if (device_check && m->nr > 0) l->run_species = std::max(l->run_species, m->ns);
     follow_density(l);
     const StepKind kind = step_kind(l, m);
     if (kind == STEP_PHASES && (rc = ensure_phase_buffers(l)) != LMB_OK) return rc;

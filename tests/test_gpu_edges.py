@@ -117,3 +117,36 @@ def test_refused_row_major_contents_do_not_run(ctx, slots, bps, what):
     assert np.array_equal(lat.get_native()[0], ref)
     lat.close()
     model.close()
+
+
+@pytest.mark.parametrize("slots,bps", [(8, 1), (16, 4)])
+def test_species_made_by_a_larger_model_are_seen_by_a_smaller_one(ctx, slots, bps):
+    """Contents checked for a model of 3 species, then run with one of 6: the
+    smaller model is refused if a species it lacks was made, and runs on if
+    none was."""
+    from lattice_microbes_b200 import _lib as L
+    from lattice_microbes_b200.solver import Lattice, Model
+    small = configs.random_problem(35, X=32, Y=8, Z=8, slots=slots, bytes_per_slot=bps, density=0.5, ns=3, nst=2, nr=3,
+                                   zeroth=False)
+    large = configs.random_problem(36, X=32, Y=8, Z=8, slots=slots, bytes_per_slot=bps, density=0.5, ns=6, nst=2)
+    large.RL[:] = 1
+    for made in (True, False):
+        if not made:
+            large.K = large.K * 0.0
+        ts, tl = oracle_tables(small), oracle_tables(large)
+        first, _, _ = oracle_run(ts, small.lattice, small.sites, 3, 0, 2)
+        mid, _, _ = oracle_run(tl, first, small.sites, 3, 2, 6)
+        particles = mid.view(np.uint8 if bps == 1 else np.uint32)
+        assert (particles.max() > 3) == made
+        ms, ml = Model.from_tables(ctx, ts), Model.from_tables(ctx, tl)
+        lat = Lattice(ctx, small.X, small.Y, small.Z, slots, bps)
+        lat.set_native(small.lattice, small.sites)
+        assert lat.run(ms, 3, 0, 2)[0] == 0
+        assert lat.run(ml, 3, 2, 6)[0] == 0
+        rc, _ = lat.run(ms, 3, 8, 2, check=False)
+        assert rc == (L.LMB_E_ARG if made else 0)
+        ref = mid if made else oracle_run(ts, mid, small.sites, 3, 8, 2)[0]
+        assert np.array_equal(lat.get_native()[0], ref)
+        lat.close()
+        ms.close()
+        ml.close()
