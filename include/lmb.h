@@ -191,6 +191,11 @@ int lmb_lattice_get_row_major(lmb_lattice *lattice, void *particles, uint8_t *si
  * (options.cmake:89-95). */
 int lmb_lattice_set_schedule(lmb_lattice *lattice, int schedule, uint32_t Ty, uint32_t Tz);
 int lmb_lattice_get_schedule(lmb_lattice *lattice, int *schedule, uint32_t *Ty, uint32_t *Tz);
+/* What the particle lists of the fused tiles hold: in the last run waited
+ * for, the tiles (times timesteps) with more particles than their list, which
+ * are worked in pieces; and the particles per site the lists are now sized
+ * for (at most the slots). */
+int lmb_lattice_tile_lists(const lmb_lattice *lattice, uint32_t *split, float *planned);
 /* Autotuner: times the per-phase schedule, the cluster-resident one where it
  * fits and the fused tile shapes with the best estimates for `timesteps` on a
  * saved copy of the lattice state, restores the state and keeps the fastest.  The

@@ -119,6 +119,7 @@ PROTOTYPES = {
     "lmb_lattice_get_row_major": (C.c_int, [vp, vp, u8p]),
     "lmb_lattice_set_schedule": (C.c_int, [vp, C.c_int, C.c_uint32, C.c_uint32]),
     "lmb_lattice_get_schedule": (C.c_int, [vp, C.POINTER(C.c_int), u32p, u32p]),
+    "lmb_lattice_tile_lists": (C.c_int, [vp, u32p, f32p]),
     "lmb_lattice_autotune": (C.c_int, [vp, vp, C.c_uint32, C.c_uint32, C.c_uint32, C.POINTER(C.c_int), u32p, u32p,
                                        f32p]),
     "lmb_lattice_device_buffers": (C.c_int, [vp, C.POINTER(vp), C.POINTER(vp)]),

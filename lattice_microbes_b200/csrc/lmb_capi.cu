@@ -89,11 +89,15 @@ struct lmb_lattice {
     // Schedule: fused tile kernel (one launch per timestep) or per-phase kernels.
     int schedule;
     TileShape tile;
-    // Particles per site when the lattice was last counted, the figure the
-    // fused plan was made for, and whether the caller left the plan to the
-    // lattice.
-    float density, plan_density;
-    bool auto_plan;
+    // Particles per site when the lattice was last counted; those of the
+    // regions that particle-list tiles could not hold (0: none, note_splits)
+    // and the mean then; the figure the fused plan was made for; whether the
+    // caller left the tile, and the schedule, to the lattice; whether its
+    // particles crowd so that the per-phase kernels serve it; tiles split in
+    // the last run.
+    float density, crowd, crowd_density, plan_density;
+    bool auto_plan, own_schedule, crowded;
+    uint32_t splits;
     // Captured timestep graphs, one per starting buffer parity, with what the
     // captured launches were given.  The table set is compared whole: the
     // kernels take it by value, and a rate change rewrites the tables in
@@ -101,7 +105,7 @@ struct lmb_lattice {
     struct Graph {
         cudaGraphExec_t exec;
         DevTables tables;
-        int schedule;
+        int schedule, kind;
         uint32_t Ty, Tz, list_smem;
         bool reaction;
         uint64_t kernels;
@@ -650,7 +654,7 @@ extern "C" int lmb_lattice_create(lmb_ctx *c, uint32_t X, uint32_t Y, uint32_t Z
         lmb_lattice_destroy(l);
         return rc;
     }
-    l->auto_plan = l->schedule == LMB_SCHEDULE_FUSED;
+    l->own_schedule = true;
     *out = l;
     return LMB_OK;
 }
@@ -684,6 +688,58 @@ static int ensure_plane_bounds(lmb_lattice *l)
     return LMB_OK;
 }
 
+// Particles per site the lists of the lattice's tiles are sized for.
+static float plan_figure(const lmb_lattice *l) { return std::max(l->density, l->crowd); }
+
+// Takes from a run's state what its particle-list tiles could not hold, for
+// the next run's plan.  Tiles split here and there cost little.  When more
+// than one tile in eight was split, the lists are sized for what the split
+// ones held, and the lattice holds at least their share of that.  These are
+// measured figures: they cannot pass the slots, however many runs split
+// tiles, and they leave zero.
+//
+// Where most timesteps split a tile and the fullest holds twice the mean or
+// more, particles crowd, and that tile alone can end every launch.  If the
+// estimate of a plan made for it is lower by a sixth or more, the lattice's
+// own plan becomes that one; and where the schedule is the lattice's own and
+// its sites are of many word planes, the per-phase kernels take it over, whose
+// time does not depend on where the particles are: sites of more than two
+// planes with plane bounds (the empty ones are skipped), of 16 without.  All
+// particles in some of the z planes, us per timestep in tiles of the mean
+// density / planned for the fullest / per-phase:
+//   IntLattice-16   128 x 128 x 64, 5 %    144 / 53..89 / 73
+//                   96 x 64 x 64, 10 %     131 / 71..91 / 51
+//                   100 x 64 x 64, 10 %    175 / 82 / 74   (no bounds)
+//   IntLattice-8    256 x 64 x 64, 10 %    120 / 61 / 65
+//                   200 x 64 x 64, 10 %    128 / 58 / 74   (no bounds)
+//   ByteLattice-16  256 x 64 x 64, 10 %    170 / 136 / 82
+//   ByteLattice-8   128^3, 6 %             69 / 56 / 88
+static void note_splits(lmb_lattice *l, const RunState &h, uint32_t n, const TileShape &t, bool auto_plan)
+{
+    l->splits = h.list_split;
+    if (!h.list_split) return;
+    const uint64_t tiles = (uint64_t)n * t.tiles_y * t.tiles_z;
+    float crowd = 0.0f;
+    if ((uint64_t)h.list_split * 8u > tiles) {
+        crowd = (float)((double)h.list_over / h.list_split / t.R);
+        l->density = std::max(l->density, crowd * (float)((double)h.list_split / (double)tiles));
+    }
+    const float most = (float)h.list_most / (float)t.R;
+    if (auto_plan && (uint64_t)h.list_split * 2u >= n && most > 2.0f * l->density && most > l->crowd) {
+        const double now = list_cost(t.tiles_y * t.tiles_z, t.R, t.list_smem, l->density, most);
+        const std::vector<TileShape> best = list_shapes(l->g, (int)l->bps, (int)l->slots, l->density, most, 1);
+        if (!best.empty() && list_cost(best[0].tiles_y * best[0].tiles_z, best[0].R, best[0].list_smem, l->density,
+                                       most) < 0.85 * now) {
+            crowd = most;
+            l->crowded = l->words > 8 || (l->pb && l->words > 2);
+        }
+    }
+    if (crowd > l->crowd) {
+        l->crowd = crowd;
+        l->crowd_density = l->density;
+    }
+}
+
 extern "C" int lmb_lattice_set_schedule(lmb_lattice *l, int schedule, uint32_t Ty, uint32_t Tz)
 {
     if (!l) return LMB_E_ARG;
@@ -692,7 +748,7 @@ extern "C" int lmb_lattice_set_schedule(lmb_lattice *l, int schedule, uint32_t T
         if (rc == LMB_OK) rc = ensure_plane_bounds(l);
         if (rc) return rc;
         l->schedule = schedule;
-        l->auto_plan = false;
+        l->auto_plan = l->own_schedule = false;
         return LMB_OK;
     }
     if (schedule == LMB_SCHEDULE_CLUSTER) {
@@ -701,7 +757,7 @@ extern "C" int lmb_lattice_set_schedule(lmb_lattice *l, int schedule, uint32_t T
         CK(cudaSetDevice(l->ctx->device));
         if (!cluster_plan(l->g, (int)l->bps, (int)l->slots, l->cap, 8 * 1024, C, P)) return LMB_E_UNSUPPORTED;
         l->schedule = schedule;
-        l->auto_plan = false;
+        l->auto_plan = l->own_schedule = false;
         return LMB_OK;
     }
     if (schedule == LMB_SCHEDULE_GRID) {
@@ -715,13 +771,14 @@ extern "C" int lmb_lattice_set_schedule(lmb_lattice *l, int schedule, uint32_t T
         if (!ok) return LMB_E_UNSUPPORTED;
         l->tile = t;
         l->schedule = schedule;
-        l->auto_plan = false;
+        l->auto_plan = l->own_schedule = false;
         return LMB_OK;
     }
     if (schedule != LMB_SCHEDULE_FUSED) return LMB_E_ARG;
     TileShape t;
-    bool ok = (Ty == 0 && Tz == 0) ? fused_default_shape(l->g, (int)l->bps, (int)l->slots, t, l->density)
-                                   : fused_make_shape(l->g, (int)l->bps, (int)l->slots, Ty, Tz, t, l->density);
+    const float density = plan_figure(l);
+    bool ok = (Ty == 0 && Tz == 0) ? fused_default_shape(l->g, (int)l->bps, (int)l->slots, t, l->density, l->crowd)
+                                   : fused_make_shape(l->g, (int)l->bps, (int)l->slots, Ty, Tz, t, density);
     if (!ok) return LMB_E_UNSUPPORTED;
     if (t.list_smem && l->words > 2) {
         const int rc = ensure_plane_bounds(l);
@@ -729,8 +786,9 @@ extern "C" int lmb_lattice_set_schedule(lmb_lattice *l, int schedule, uint32_t T
     }
     l->tile = t;
     l->schedule = schedule;
-    l->plan_density = l->density;
+    l->plan_density = density;
     l->auto_plan = Ty == 0 && Tz == 0;
+    l->own_schedule = false;
     return LMB_OK;
 }
 
@@ -741,6 +799,14 @@ extern "C" int lmb_lattice_get_schedule(lmb_lattice *l, int *schedule, uint32_t 
     const bool tiled = l->schedule == LMB_SCHEDULE_FUSED || l->schedule == LMB_SCHEDULE_GRID;
     if (Ty) *Ty = tiled ? l->tile.Ty : 0;
     if (Tz) *Tz = tiled ? l->tile.Tz : 0;
+    return LMB_OK;
+}
+
+extern "C" int lmb_lattice_tile_lists(const lmb_lattice *l, uint32_t *split, float *planned)
+{
+    if (!l) return LMB_E_ARG;
+    if (split) *split = l->splits;
+    if (planned) *planned = l->plan_density;
     return LMB_OK;
 }
 
@@ -917,13 +983,14 @@ static uint32_t *plane_bounds(lmb_lattice *l, int b) { return l->pb ? l->pb + (s
 // The kernels that run a timestep of the lattice's schedule: the
 // particle-list kernel where its tile fits and its list entries hold the
 // model's species ids, the dense fused kernel where they do not, and the
-// per-phase kernels for PHASES and for a tile that only the particle-list
-// kernel could hold.
+// per-phase kernels for PHASES, for a tile that only the particle-list
+// kernel could hold, and for a lattice of its own schedule whose particles
+// crowd (note_splits).
 enum StepKind { STEP_LIST, STEP_DENSE, STEP_PHASES };
 
 static StepKind step_kind(const lmb_lattice *l, const lmb_model *m)
 {
-    if (l->schedule != LMB_SCHEDULE_FUSED) return STEP_PHASES;
+    if (l->schedule != LMB_SCHEDULE_FUSED || (l->own_schedule && l->crowded)) return STEP_PHASES;
     if (l->tile.list_smem && (l->bps == 1 || m->ns <= LIST_MAX_SPECIES)) return STEP_LIST;
     return l->tile.dense ? STEP_DENSE : STEP_PHASES;
 }
@@ -946,12 +1013,13 @@ static cudaError_t launch_fused_step(lmb_lattice *l, const lmb_model *m, cudaStr
 static void follow_density(lmb_lattice *l)
 {
     if (l->schedule != LMB_SCHEDULE_FUSED) return;
-    if (l->density <= 1.02f * l->plan_density && l->density >= 0.8f * l->plan_density) return;
+    const float density = plan_figure(l);
+    if (density <= 1.02f * l->plan_density && density >= 0.8f * l->plan_density) return;
     TileShape t;
-    if (l->auto_plan ? fused_default_shape(l->g, (int)l->bps, (int)l->slots, t, l->density)
-                     : fused_make_shape(l->g, (int)l->bps, (int)l->slots, l->tile.Ty, l->tile.Tz, t, l->density))
+    if (l->auto_plan ? fused_default_shape(l->g, (int)l->bps, (int)l->slots, t, l->density, l->crowd)
+                     : fused_make_shape(l->g, (int)l->bps, (int)l->slots, l->tile.Ty, l->tile.Tz, t, density))
         l->tile = t;
-    l->plan_density = l->density;
+    l->plan_density = density;
 }
 
 // Queues one timestep (schedule of the lattice) and flips the buffer index.
@@ -1001,8 +1069,9 @@ static cudaError_t reset_plane_bounds(lmb_lattice *l, const lmb_model *m, cudaSt
 static int ensure_graph(lmb_lattice *l, lmb_model *m)
 {
     lmb_lattice::Graph &gr = l->graph[l->cur];
+    const int kind = step_kind(l, m);
     const bool same = gr.exec && memcmp(&gr.tables, &m->dev, sizeof(DevTables)) == 0 && gr.schedule == l->schedule &&
-                      gr.Ty == l->tile.Ty && gr.Tz == l->tile.Tz && gr.list_smem == l->tile.list_smem &&
+                      gr.kind == kind && gr.Ty == l->tile.Ty && gr.Tz == l->tile.Tz && gr.list_smem == l->tile.list_smem &&
                       gr.reaction == (m->nr > 0);
     if (same) return LMB_OK;
     if (gr.exec) {
@@ -1035,6 +1104,7 @@ static int ensure_graph(lmb_lattice *l, lmb_model *m)
     }
     memcpy(&gr.tables, &m->dev, sizeof(DevTables));
     gr.schedule = l->schedule;
+    gr.kind = kind;
     gr.Ty = l->tile.Ty;
     gr.Tz = l->tile.Tz;
     gr.list_smem = l->tile.list_smem;
@@ -1061,6 +1131,8 @@ static int validate_for_model(lmb_lattice *l, const lmb_model *m)
         l->max_species = l->rs_host->max_species;
         l->max_site_type = l->rs_host->max_site_type;
         l->density = (float)((double)l->rs_host->occupied / l->g.N);
+        l->crowd = 0.0f;
+        l->crowded = false;
         l->validated = true;
         l->run_species = 0;
     }
@@ -1230,16 +1302,18 @@ extern "C" int lmb_run_wait(lmb_lattice *l, lmb_run_stats *st)
     const bool refused = l->pending_check && h.status == LMB_E_ARG;
     if (l->pending_check) {
         // The device's check of the contents, kept as the host's would be.
+        // Contents of the same density are taken to crowd as those before.
         l->max_species = h.max_species;
         l->max_site_type = h.max_site_type;
         l->density = (float)((double)h.occupied / l->g.N);
+        if (std::fabs(l->density - l->crowd_density) > 0.25f * l->crowd_density) {
+            l->crowd = 0.0f;
+            l->crowded = false;
+        }
         l->validated = true;
         l->pending_check = false;
     }
-    // Tiles split here and there cost little; a list too short for one tile
-    // in eight is sized anew.
-    if ((uint64_t)h.list_split * 8u > (uint64_t)l->pending_n * l->tile.tiles_y * l->tile.tiles_z)
-        l->density = std::max(l->density, l->plan_density) * 1.5f;
+    note_splits(l, h, l->pending_n, l->tile, l->auto_plan);
     if (refused) {
         // Refused before the first timestep: the lattice is where it was.
         done = 0;
@@ -1392,19 +1466,69 @@ extern "C" int lmb_lattice_autotune(lmb_lattice *l, const lmb_model *m, uint32_t
     const int cur0 = l->cur;
     const int sched0 = l->schedule;
     const TileShape tile0 = l->tile;
-    const bool auto0 = l->auto_plan;
+    const bool auto0 = l->auto_plan, own0 = l->own_schedule, crowded0 = l->crowded;
     struct Cand { int sched; uint32_t ty, tz; };
-    std::vector<Cand> cands = {{LMB_SCHEDULE_PHASES, 0, 0}, {LMB_SCHEDULE_CLUSTER, 0, 0}};
-    // Fused: the eight particle-list tiles with the best estimates; every
-    // dense tile where no particle-list one fits.
     int rc = validate_for_model(l, m);
     if (rc != LMB_OK) {
         cudaFree(save);
         return rc;
     }
-    for (const TileShape &t : list_shapes(l->g, (int)l->bps, (int)l->slots, l->density, 8))
-        cands.push_back({LMB_SCHEDULE_FUSED, t.Ty, t.Tz});
-    if (cands.size() == 2) {
+    const float plan0 = l->plan_density, density0 = l->density, crowd0 = l->crowd;
+    cudaEvent_t e0, e1;
+    cudaEventCreate(&e0);
+    cudaEventCreate(&e1);
+    // One run from the saved state, in the schedule set.
+    auto trial = [&](float &ms) {
+        l->cur = cur0;
+        cudaMemcpyAsync(l->buf[l->cur], save, wbytes, cudaMemcpyDeviceToDevice, c->stream);
+        cudaEventRecord(e0, c->stream);
+        int status = lmb_run_async(l, m, seed, first, timesteps, LMB_OVERFLOW_CLASSIC);
+        if (status != LMB_OK) return status;
+        cudaEventRecord(e1, c->stream);
+        lmb_run_stats st;
+        status = lmb_run_wait(l, &st);
+        ms = 0;
+        if (status == LMB_OK) cudaEventElapsedTime(&ms, e0, e1);
+        return status;
+    };
+    float ms = 0, best = 1e30f;
+    Cand bestc = {sched0, tile0.Ty, tile0.Tz};
+    // A candidate's warm-up run and its timed one.  Each starts from the
+    // lattice's own figures; what its warm-up could not hold sizes the list of
+    // its timed run, and the best one's list stays.
+    float best_crowd = crowd0;
+    auto time_candidate = [&](const Cand &cd) {
+        l->density = density0;
+        if (lmb_lattice_set_schedule(l, cd.sched, cd.ty, cd.tz) != LMB_OK) return;
+        for (int rep = 0; rep < 2 && rc == LMB_OK; rep++) {
+            const float crowd = l->crowd;
+            rc = trial(ms);
+            if (rc != LMB_OK && resident_schedule(cd.sched) && rc == LMB_E_CUDA) {
+                // A cluster the device would not launch: not a candidate.
+                cudaGetLastError();
+                rc = LMB_OK;
+                break;
+            }
+            if (rc == LMB_OK && rep == 1 && ms < best) {
+                best = ms;
+                lmb_lattice_get_schedule(l, &bestc.sched, &bestc.ty, &bestc.tz);
+                best_crowd = crowd;
+            }
+        }
+    };
+    // Fused: the lattice's own plan first, whose warm-up shows whether its
+    // particles crowd; the particle-list tiles with the best estimates, eight
+    // in all, made for the fullest where they do; every dense tile where no
+    // particle-list one fits.
+    std::vector<Cand> cands;
+    float crowd1 = crowd0;
+    if (!list_shapes(l->g, (int)l->bps, (int)l->slots, l->density, l->crowd, 1).empty()) {
+        time_candidate({LMB_SCHEDULE_FUSED, 0, 0});
+        crowd1 = l->crowd;
+        const uint32_t own_y = l->tile.Ty, own_z = l->tile.Tz;
+        for (const TileShape &t : list_shapes(l->g, (int)l->bps, (int)l->slots, density0, crowd1, 8))
+            if ((t.Ty != own_y || t.Tz != own_z) && cands.size() < 7) cands.push_back({LMB_SCHEDULE_FUSED, t.Ty, t.Tz});
+    } else {
         const uint32_t dims[] = {1, 2, 4, 8, 16};
         for (uint32_t ty : dims)
             for (uint32_t tz : dims) {
@@ -1416,38 +1540,12 @@ extern "C" int lmb_lattice_autotune(lmb_lattice *l, const lmb_model *m, uint32_t
     // LMB_SCHEDULE_GRID is not a candidate: on one lattice it times as its
     // fused plan does, and its cooperative launch cannot overlap another
     // lattice's run on a second stream, as fused launches do.
-    cudaEvent_t e0, e1;
-    cudaEventCreate(&e0);
-    cudaEventCreate(&e1);
-    float best = 1e30f;
-    Cand bestc = {sched0, tile0.Ty, tile0.Tz};
+    cands.push_back({LMB_SCHEDULE_PHASES, 0, 0});
+    cands.push_back({LMB_SCHEDULE_CLUSTER, 0, 0});
     for (const Cand &cd : cands) {
-        if (lmb_lattice_set_schedule(l, cd.sched, cd.ty, cd.tz) != LMB_OK) continue;
-        // warm-up launch, then the timed one, each from the saved state
-        for (int rep = 0; rep < 2 && rc == LMB_OK; rep++) {
-            l->cur = cur0;
-            cudaMemcpyAsync(l->buf[l->cur], save, wbytes, cudaMemcpyDeviceToDevice, c->stream);
-            cudaEventRecord(e0, c->stream);
-            rc = lmb_run_async(l, m, seed, first, timesteps, LMB_OVERFLOW_CLASSIC);
-            if (rc != LMB_OK && resident_schedule(cd.sched) && rc == LMB_E_CUDA) {
-                // A cluster the device would not launch: not a candidate.
-                cudaGetLastError();
-                rc = LMB_OK;
-                break;
-            }
-            if (rc != LMB_OK) break;
-            cudaEventRecord(e1, c->stream);
-            lmb_run_stats st;
-            rc = lmb_run_wait(l, &st);
-            if (rc != LMB_OK) break;
-            float ms = 0;
-            cudaEventElapsedTime(&ms, e0, e1);
-            if (rep == 1 && ms < best) {
-                best = ms;
-                bestc = cd;
-            }
-        }
         if (rc != LMB_OK) break;
+        l->crowd = crowd1;
+        time_candidate(cd);
     }
     cudaEventDestroy(e0);
     cudaEventDestroy(e1);
@@ -1459,8 +1557,15 @@ extern "C" int lmb_lattice_autotune(lmb_lattice *l, const lmb_model *m, uint32_t
         l->schedule = sched0;
         l->tile = tile0;
         l->auto_plan = auto0;
+        l->own_schedule = own0;
+        l->crowd = crowd0;
+        l->crowded = crowded0;
+        l->density = density0;
+        l->plan_density = plan0;
         return rc;
     }
+    l->crowd = best_crowd;
+    l->density = density0;
     lmb_lattice_set_schedule(l, bestc.sched, bestc.ty, bestc.tz);
     if (schedule) *schedule = bestc.sched;
     if (Ty) *Ty = bestc.ty;
@@ -1561,7 +1666,7 @@ static int batch_check_members(lmb_ctx *c, uint32_t count, lmb_lattice *const *l
         if (!l || !m || l->ctx != c || m->ctx != c) return LMB_E_ARG;
         if ((int)l->bps != bps || (int)l->slots != slots) return LMB_E_ARG;
         if (m->has_desc && (m->X != l->g.X || m->Y != l->g.Y || m->Z != l->g.Z)) return LMB_E_ARG;
-        if (list && (!fused_batch_shape(l->g, bps, slots, true, l->density, plan[j]) ||
+        if (list && (!fused_batch_shape(l->g, bps, slots, true, plan_figure(l), plan[j]) ||
                      (bps != 1 && m->ns > LIST_MAX_SPECIES)))
             list = false;
     }
@@ -1578,7 +1683,7 @@ static int batch_set(lmb_batch *b, uint32_t count, lmb_lattice *const *lattices,
     for (uint32_t j = 0; j < count; j++) {
         const auto it = b->tuned.find(size_key(lattices[j]->g));
         TileShape t;
-        if (it != b->tuned.end() && fused_batch_shape_ok(lattices[j]->g, b->bps, b->slots, list, lattices[j]->density,
+        if (it != b->tuned.end() && fused_batch_shape_ok(lattices[j]->g, b->bps, b->slots, list, plan_figure(lattices[j]),
                                                          it->second.first, it->second.second, t))
             plan[j] = t;
     }
@@ -1684,8 +1789,9 @@ static int batch_prepare(lmb_batch *b)
             // last run, new contents), in the member's tile while it fits.
             TileShape t;
             const TileShape &p = b->tiles[j];
-            if (fused_batch_shape_ok(l->g, b->bps, b->slots, true, l->density, p.Ty, p.Tz, t) ||
-                fused_batch_shape(l->g, b->bps, b->slots, true, l->density, t))
+            const float density = plan_figure(l);
+            if (fused_batch_shape_ok(l->g, b->bps, b->slots, true, density, p.Ty, p.Tz, t) ||
+                fused_batch_shape(l->g, b->bps, b->slots, true, density, t))
                 b->tiles[j] = t;
         }
         FusedJob &jb = b->jobs_host[j];
@@ -1831,8 +1937,7 @@ extern "C" int lmb_batch_wait(lmb_batch *b, lmb_run_stats *stats)
         lmb_lattice *l = b->lats[j];
         const uint32_t done = h.status == LMB_OK ? b->pending_n[j] : h.failed_step - b->pending_first[j];
         l->cur = b->cur0[j] ^ (int)((h.status == LMB_OK ? done : done + 1) & 1u);
-        if ((uint64_t)h.list_split * 8u > (uint64_t)b->pending_n[j] * b->tiles[j].tiles_y * b->tiles[j].tiles_z)
-            l->density *= 1.5f;
+        note_splits(l, h, b->pending_n[j], b->tiles[j], false);
         if (stats) {
             stats[j].status = h.status;
             stats[j].steps_done = done;
@@ -1927,7 +2032,9 @@ extern "C" int lmb_batch_autotune(lmb_batch *b, const uint32_t *seeds, uint32_t 
         for (uint32_t Ty : cands)
             for (uint32_t Tz : cands) {
                 TileShape t;
-                if (!fused_batch_shape_ok(g, b->bps, b->slots, b->list, b->lats[members[0]]->density, Ty, Tz, t)) continue;
+                if (!fused_batch_shape_ok(g, b->bps, b->slots, b->list, plan_figure(b->lats[members[0]]), Ty, Tz,
+                                          t))
+                    continue;
                 if (t.Ty == keep.Ty && t.Tz == keep.Tz) continue;
                 for (uint32_t j : members) b->tiles[j] = t;
                 const float ms = trial();

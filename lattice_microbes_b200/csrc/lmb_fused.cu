@@ -618,14 +618,15 @@ bool fused_make_shape(const Geometry &g, int bps, int slots, uint32_t Ty, uint32
 // edges such as 60, 72 or 96 be cut into as many tiles as are resident.
 static const uint32_t LIST_EDGES[] = {1, 2, 3, 4, 5, 6, 7, 8, 9, 10, 12, 14, 16};
 
-std::vector<TileShape> list_shapes(const Geometry &g, int bps, int slots, float density, size_t most)
+std::vector<TileShape> list_shapes(const Geometry &g, int bps, int slots, float density, float crowd, size_t most)
 {
+    const float held = std::max(density, crowd);
     std::vector<std::pair<double, TileShape>> found;
     for (uint32_t Ty : LIST_EDGES)
         for (uint32_t Tz : LIST_EDGES) {
             TileShape t;
-            if (!fused_make_shape(g, bps, slots, Ty, Tz, t, density) || !t.list_fits) continue;
-            found.push_back({list_cost(t.tiles_y * t.tiles_z, t.R, t.list_smem, density), t});
+            if (!fused_make_shape(g, bps, slots, Ty, Tz, t, held) || !t.list_fits) continue;
+            found.push_back({list_cost(t.tiles_y * t.tiles_z, t.R, t.list_smem, density, crowd), t});
         }
     std::stable_sort(found.begin(), found.end(), [](const auto &a, const auto &b) { return a.first < b.first; });
     std::vector<TileShape> out;
@@ -636,9 +637,9 @@ std::vector<TileShape> list_shapes(const Geometry &g, int bps, int slots, float 
 // Default plan: the cheapest particle-list tile; where none fits, the dense
 // tile with the least halo overhead among those that still give every SM two
 // blocks, failing that, the most blocks.
-bool fused_default_shape(const Geometry &g, int bps, int slots, TileShape &ts, float density)
+bool fused_default_shape(const Geometry &g, int bps, int slots, TileShape &ts, float density, float crowd)
 {
-    const std::vector<TileShape> list = list_shapes(g, bps, slots, density, 1);
+    const std::vector<TileShape> list = list_shapes(g, bps, slots, density, crowd, 1);
     if (!list.empty()) {
         ts = list[0];
         return true;

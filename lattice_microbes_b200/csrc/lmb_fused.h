@@ -63,8 +63,10 @@ cudaError_t launch_fused_batch(int bytes_per_slot, int slots, const FusedJob *jo
 // density: particles per site the list of a particle-list tile is sized for.
 bool fused_make_shape(const Geometry &g, int bytes_per_slot, int slots, uint32_t Ty, uint32_t Tz, TileShape &ts,
                       float density = LIST_DEFAULT_DENSITY);
+// crowd: particles per site of the fullest region, where particles crowd (0:
+// spread evenly).
 bool fused_default_shape(const Geometry &g, int bytes_per_slot, int slots, TileShape &ts,
-                         float density = LIST_DEFAULT_DENSITY);
+                         float density = LIST_DEFAULT_DENSITY, float crowd = 0.0f);
 // list: for the particle-list batch kernel, otherwise for the dense one.
 bool fused_batch_shape(const Geometry &g, int bytes_per_slot, int slots, bool list, float density, TileShape &ts);
 bool fused_batch_shape_ok(const Geometry &g, int bytes_per_slot, int slots, bool list, float density, uint32_t Ty,
@@ -82,11 +84,13 @@ cudaError_t launch_fused(int bytes_per_slot, int slots, const uint32_t *src, uin
 size_t list_smem_bytes(const Geometry &g, int bytes_per_slot, int slots, uint32_t Ty, uint32_t Tz, float density,
                        bool &fits);
 void list_fill_shape(const Geometry &g, TileShape &ts);
-// Estimated SM cycles of a timestep with `tiles` tiles of R region sites.
-double list_cost(uint32_t tiles, uint32_t R, size_t smem, float density);
+// Estimated SM cycles of a timestep with `tiles` tiles of R region sites, the
+// fullest with `crowd` particles per site (0: as the others).
+double list_cost(uint32_t tiles, uint32_t R, size_t smem, float density, float crowd = 0.0f);
 // The particle-list tiles of a lattice, cheapest estimate first (at most
 // `most` of them).
-std::vector<TileShape> list_shapes(const Geometry &g, int bytes_per_slot, int slots, float density, size_t most);
+std::vector<TileShape> list_shapes(const Geometry &g, int bytes_per_slot, int slots, float density, float crowd,
+                                   size_t most);
 cudaError_t launch_list(int bytes_per_slot, int slots, const uint32_t *src, uint32_t *dst, const uint8_t *sites,
                         const Geometry &g, const DevTables &m, RunState *rs, OverflowEntry *queue, uint32_t cap,
                         const TileShape &ts, int with_reaction, const uint32_t *pb_src, uint32_t *pb_dst,

@@ -2,6 +2,7 @@
 #pragma once
 
 #include <cuda_runtime.h>
+#include <stddef.h>
 #include <stdint.h>
 
 #include <atomic>
@@ -93,7 +94,7 @@ struct RunState {
     alignas(8) uint32_t tiles_done;  // fused kernels: blocks finished in this launch
     uint32_t ovf_count;              // entries in the overflow list, carried ones first
     uint32_t rx_count;    // per-phase schedule: sites the z sweep listed for the reaction step
-    uint32_t list_split;  // particle-list kernel: times a tile of this run had more particles than its list holds
+    uint32_t list_split;  // particle-list kernel: tiles of this run whose region had more particles than their list holds
     uint32_t rx_skip;     // timesteps left to run without the list (it overflowed recently)
     // timestep_hash(seed, step, k) for the sub-steps k = 0..3 of `step`, set
     // with every change of step (the per-phase kernels read them here).
@@ -110,7 +111,12 @@ struct RunState {
     // flags of the timesteps, by timestep index modulo 3.
     unsigned long long grid_bar;
     uint32_t grid_full[3];
+    // The most particles of a split tile's region, and the sum over them
+    // (last: what every kernel reads stays in the first 128 bytes).
+    uint32_t list_most;
+    unsigned long long list_over;
 };
+static_assert(offsetof(RunState, th) + sizeof(RunState::th) <= 128, "the run state's hot words share a line");
 
 
 // tiles_done | ovf_count << 32, for 64-bit atomics (every kernel adds to

@@ -711,7 +711,8 @@ __global__ void begin_run_kernel(RunState *rs, uint32_t seed, uint32_t first, ui
     rs->overflows = 0;
     rs->reactions = 0;
     rs->tiles_done = 0;
-    rs->list_split = 0;
+    rs->list_split = rs->list_most = 0;
+    rs->list_over = 0;
     rs->rx_count = 0;
     rs->rx_skip = 0;
     if (mode == LMB_OVERFLOW_CLASSIC) {
@@ -763,7 +764,8 @@ __global__ void begin_batch_kernel(RunState *const *rs_ptrs, const uint32_t *see
     rs->overflows = 0;
     rs->reactions = 0;
     rs->tiles_done = 0;
-    rs->list_split = 0;
+    rs->list_split = rs->list_most = 0;
+    rs->list_over = 0;
     rs->rx_count = 0;
     rs->rx_skip = 0;
     if (mode == LMB_OVERFLOW_CLASSIC) {

@@ -818,7 +818,11 @@ __device__ __forceinline__ void list_tile(const uint32_t *__restrict__ src, uint
             // list for more): a smaller sub-tile from the same corner.  z
             // first, then y (with one z plane, so that y pieces only ever
             // split a single plane of rows).
-            if (tid == 0) atomicAdd(&rs->list_split, 1u);
+            if (tid == 0 && t.R == ts.R) {
+                atomicAdd(&rs->list_split, 1u);
+                atomicAdd(&rs->list_over, (unsigned long long)n);
+                atomicMax(&rs->list_most, n);
+            }
             if (t.y0 == 0 && t.ctz > 1u) {
                 t.ctz = (t.ctz + 1u) / 2u;
             } else if (t.cty > 1u) {
@@ -971,17 +975,20 @@ static uint32_t list_threads(uint32_t R, size_t smem)
 // lattices: about 5 instructions per region site and 15 per region particle,
 // an SM's rate growing with its resident warps towards 3 per cycle, a floor of
 // 6000 cycles for a block's chain of passes; waves of 148 SMs.
-double list_cost(uint32_t tiles, uint32_t R, size_t smem, float density)
+// Where particles crowd, the launch lasts at least as long as its fullest
+// tile, whose SM's other tiles are soon done.
+double list_cost(uint32_t tiles, uint32_t R, size_t smem, float density, float crowd)
 {
     const uint32_t warps = list_threads(R, smem) / 32u, fit = list_blocks_fit(smem);
     const uint32_t per_sm = std::max(1u, std::min(fit, 32u / warps));  // blocks an SM holds
-    const double instr = 3000.0 + (5.1 + 15.1 * (double)density) * (double)R;
-    auto wave = [&](uint32_t blocks) {
+    auto wave = [&](uint32_t blocks, float d) {
+        const double instr = 3000.0 + (5.1 + 15.1 * (double)d) * (double)R;
         const double w = (double)(warps * blocks), rate = 3.0 * w / (w + 14.0);
         return std::max(6000.0, blocks * instr / rate);
     };
     const uint32_t slots = 148u * per_sm, full = tiles / slots, rest = tiles - full * slots;
-    return full * wave(per_sm) + (rest ? wave((rest + 147u) / 148u) : 0.0);
+    const double even = full * wave(per_sm, density) + (rest ? wave((rest + 147u) / 148u, density) : 0.0);
+    return crowd > density ? std::max(even, wave(1u, crowd)) : even;
 }
 
 void list_fill_shape(const Geometry &g, TileShape &ts)

@@ -188,6 +188,13 @@ class Lattice:
         L.check(L.lib().lmb_lattice_get_schedule(self.handle, C.byref(s), C.byref(ty), C.byref(tz)))
         return s.value, ty.value, tz.value
 
+    def tile_lists(self):
+        """(tiles of the last run whose particles did not fit their list,
+        particles per site the lists are sized for)."""
+        n, d = C.c_uint32(), C.c_float()
+        L.check(L.lib().lmb_lattice_tile_lists(self.handle, C.byref(n), C.byref(d)))
+        return n.value, d.value
+
     def autotune(self, model, seed, first_timestep, timesteps):
         s, ty, tz, ms = C.c_int(), C.c_uint32(), C.c_uint32(), C.c_float()
         L.check(L.lib().lmb_lattice_autotune(self.handle, model.handle, seed, first_timestep, timesteps,

@@ -188,3 +188,91 @@ def test_zeroth_order_rate_switched_on_between_runs(ctx, slots, bps):
         assert np.array_equal(out, ref), piece
         lat.close()
         model.close()
+
+
+def _tiles(lat):
+    _, Ty, Tz = lat.schedule()
+    return (lat.Y // Ty) * (lat.Z // Tz)
+
+
+def test_lists_follow_a_lattice_that_fills_up(ctx):
+    """An empty lattice with sources: its tiles start with the shortest
+    lists and are split as it fills, and the lists are sized anew from what
+    the split tiles held, not from the count of 0."""
+    from lattice_microbes_b200.solver import Lattice, Model
+    spec = configs.random_problem(81, X=64, Y=32, Z=32, density=0.0)
+    spec.K = np.where(spec.rtype == configs.ZEROTH, 0.004 * spec.nsites, 0.0)
+    spec.RL[:] = 1
+    t = oracle_tables(spec)
+    model = Model.from_tables(ctx, t)
+    lat = Lattice(ctx, spec.X, spec.Y, spec.Z, 8, 1)
+    lat.set_native(spec.lattice, spec.sites)
+    seen = []
+    for k in range(10):
+        assert lat.run(model, 3, 16 * k, 16)[0] == 0
+        seen.append(lat.tile_lists())
+    ref, rc, _ = oracle_run(t, spec.lattice, spec.sites, 3, 0, 160)
+    assert rc == 0
+    assert np.array_equal(lat.get_native()[0], ref)
+    density = np.count_nonzero(ref.view(np.uint8)) / spec.nsites
+    assert max(s for s, _ in seen) > 0, seen
+    assert seen[-1][0] * 8 <= 16 * _tiles(lat), seen
+    assert density / 2 < seen[-1][1] <= 8, (density, seen)
+    lat.close()
+    model.close()
+
+
+@pytest.mark.parametrize("slots,bps", [(8, 1), (16, 4)])
+@pytest.mark.parametrize("tile", [None, (0, 0), (8, 8)])
+def test_lists_of_a_crowded_corner_stay_bounded(ctx, slots, bps, tile):
+    """Full sites in one corner, in the lattice's own schedule and plan, in the
+    fused schedule's own plan and in a tile that cannot hold them: the figure
+    the lists are sized for is a measured one, however many runs split tiles,
+    and an autotuner's trials leave none that is not."""
+    from lattice_microbes_b200 import _lib as L
+    from lattice_microbes_b200.solver import Lattice, Model
+    spec = configs.random_problem(82, X=64, Y=64, Z=64, slots=slots, bytes_per_slot=bps, density=0.0, nr=0, nst=1,
+                                  qmax=0.002)
+    N = spec.nsites
+    rng = np.random.default_rng(4)
+    z, y, x = np.meshgrid(np.arange(6), np.arange(24), np.arange(64), indexing="ij")
+    at = (x + y * spec.X + z * spec.X * spec.Y).reshape(-1)
+    lattice = np.zeros_like(spec.lattice)
+    for k in range(slots - 2):
+        sp = rng.integers(1, spec.ns + 1, at.size).astype(np.uint32)
+        if bps == 1:
+            lattice[(k // 4) * N + at] |= sp << np.uint32(8 * (k % 4))
+        else:
+            lattice[k * N + at] = sp
+    t = oracle_tables(spec)
+    model = Model.from_tables(ctx, t)
+    lat = Lattice(ctx, spec.X, spec.Y, spec.Z, slots, bps)
+    if tile:
+        lat.set_schedule(L.LMB_SCHEDULE_FUSED, *tile)
+    lat.set_native(lattice, spec.sites)
+    seen = []
+    for k in range(12):
+        assert lat.run(model, 3, 2 * k, 2)[0] == 0
+        seen.append(lat.tile_lists())
+    ref, rc, _ = oracle_run(t, lattice, spec.sites, 3, 0, 24)
+    assert rc == 0
+    assert np.array_equal(lat.get_native()[0], ref)
+    assert max(s for s, _ in seen) > 0, seen
+    assert all(d <= slots for _, d in seen), seen
+    if tile != (8, 8):
+        assert seen[-1][0] == 0, seen
+    # Crowded contents of an IntLattice go to the per-phase kernels when the
+    # schedule is the lattice's own; even contents come back to the tiles.
+    _, _, launches = lat.run_profiled(model, 3, 24, 2)
+    assert (launches[5] == 0) == (tile is None and bps == 4)
+    even = np.zeros_like(lattice)
+    even[::37] = 1
+    lat.set_native(even, spec.sites)
+    assert lat.run_profiled(model, 3, 26, 2)[2][5] == 2
+    assert np.array_equal(lat.get_native()[0], oracle_run(t, even, spec.sites, 3, 26, 2)[0])
+    lat.set_native(lattice, spec.sites)
+    lat.autotune(model, 3, 24, 4)
+    lat.set_schedule(L.LMB_SCHEDULE_FUSED)
+    assert lat.tile_lists()[1] <= slots
+    lat.close()
+    model.close()
