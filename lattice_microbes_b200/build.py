@@ -17,7 +17,8 @@ LIB = os.path.join(PKG, "liblmb200.so")
 
 SOURCES = ["lmb_kernels.cu", "lmb_fused.cu", "lmb_list.cu", "lmb_capi.cu", "lmb_noalloc.cu", "lmb_cme.cu",
            "lmb_serve.cu", "lmb_lmfile.cu"]
-HEADERS = ["lmb_internal.h", "lmb_device.cuh", "lmb_site.cuh", "lmb_overflow.cuh", "lmb_fused.h", "lmb_stage.cuh"]
+HEADERS = ["lmb_internal.h", "lmb_device.cuh", "lmb_site.cuh", "lmb_overflow.cuh", "lmb_fused.h", "lmb_stage.cuh",
+           "lmb_smem.h"]
 
 NVCC_FLAGS = [
     "-gencode", "arch=compute_100a,code=sm_100a",

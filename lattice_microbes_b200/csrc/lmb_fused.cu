@@ -665,25 +665,6 @@ bool fused_default_shape(const Geometry &g, int bps, int slots, TileShape &ts, f
     return found;
 }
 
-// The dynamic shared-memory limit is raised once per instantiation (per
-// device) to the largest size any launch needs; setting it on every launch
-// costs host time comparable to the kernel itself.
-template <int BPS, int S, int MINB>
-static cudaError_t ensure_smem_limit(size_t smem)
-{
-    static size_t granted[64] = {0};
-    int dev = 0;
-    cudaGetDevice(&dev);
-    if (dev < 0 || dev >= 64) return cudaErrorInvalidDevice;
-    // The kernel's static shared memory counts against the default 48 KB
-    // too, so the limit is raised for any size not granted yet.
-    if (smem <= granted[dev]) return cudaSuccess;
-    cudaError_t e = cudaFuncSetAttribute(fused_step_kernel<BPS, S, MINB>,
-                                         cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    if (e == cudaSuccess) granted[dev] = smem;
-    return e;
-}
-
 // A tile a batch may use: it fits, and its region leaves room for the two
 // blocks per SM the batch kernels are built for.
 bool fused_batch_shape_ok(const Geometry &g, int bps, int slots, bool list, float density, uint32_t Ty, uint32_t Tz,
@@ -726,7 +707,7 @@ static cudaError_t fused_launch(dim3 grid, dim3 block, size_t smem, cudaStream_t
                                 RunState *rs, OverflowEntry *list, uint32_t cap, const TileShape &ts,
                                 int with_reaction)
 {
-    cudaError_t e = ensure_smem_limit<BPS, S, MINB>(smem);
+    cudaError_t e = raise_smem_limit<fused_step_kernel<BPS, S, MINB>>(smem);
     if (e != cudaSuccess) return e;
     return launch_chain(fused_step_kernel<BPS, S, MINB>, grid, block, smem, stream, src, dst, sites, g, m, rs, list,
                         cap, ts, with_reaction);
@@ -764,25 +745,9 @@ cudaError_t launch_fused(int bps, int slots, const uint32_t *src, uint32_t *dst,
     return cudaErrorInvalidValue;
 }
 
-template <int BPS, int S>
-static cudaError_t ensure_batch_smem_limit(size_t smem)
-{
-    static size_t granted[64] = {0};
-    int dev = 0;
-    cudaGetDevice(&dev);
-    if (dev < 0 || dev >= 64) return cudaErrorInvalidDevice;
-    // The kernel's static shared memory counts against the default 48 KB
-    // too, so the limit is raised for any size not granted yet.
-    if (smem <= granted[dev]) return cudaSuccess;
-    cudaError_t e = cudaFuncSetAttribute(fused_batch_kernel<BPS, S>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                         (int)smem);
-    if (e == cudaSuccess) granted[dev] = smem;
-    return e;
-}
-
 #define BATCH_DISPATCH(BPS_, S_)                                                                      \
     if (bps == BPS_ && slots == S_) {                                                                 \
-        cudaError_t e = ensure_batch_smem_limit<BPS_, S_>(smem);                                      \
+        cudaError_t e = raise_smem_limit<fused_batch_kernel<BPS_, S_>>(smem);                         \
         if (e != cudaSuccess) return e;                                                               \
         return launch_chain(fused_batch_kernel<BPS_, S_>, dim3(total_tiles), dim3(FUSED_THREADS), smem, stream, \
                             jobs, njobs, parity);                                                     \
@@ -1029,8 +994,7 @@ static bool cluster_plan_t(const Geometry &g, uint32_t cap, uint32_t stage_bytes
         cluster_layout(g, W, p, cap, wa, ta);
         const size_t sm = ta + stage_bytes;
         if (sm > 200 * 1024) continue;
-        if (cudaFuncSetAttribute(cluster_run_kernel<BPS, S>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm) !=
-                cudaSuccess ||
+        if (raise_smem_limit<cluster_run_kernel<BPS, S>>(sm) != cudaSuccess ||
             cudaFuncSetAttribute(cluster_run_kernel<BPS, S>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) !=
                 cudaSuccess) {
             cudaGetLastError();
@@ -1234,21 +1198,9 @@ __global__ void __launch_bounds__(FUSED_THREADS, 2)
 template <int BPS, int S>
 static uint32_t grid_blocks_per_sm(size_t smem)
 {
-    // The limit only grows (per device), as for the fused kernel, so that a
-    // smaller plan checked later never lowers it under a larger one's launch.
-    static size_t granted[64] = {0};
-    int dev = 0;
-    if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) {
+    if (raise_smem_limit<fused_grid_kernel<BPS, S>>(smem) != cudaSuccess) {
         cudaGetLastError();
         return 0;
-    }
-    if (smem > granted[dev]) {
-        if (cudaFuncSetAttribute(fused_grid_kernel<BPS, S>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) !=
-            cudaSuccess) {
-            cudaGetLastError();
-            return 0;
-        }
-        granted[dev] = smem;
     }
     int per_sm = 0;
     if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fused_grid_kernel<BPS, S>, FUSED_THREADS, smem) !=

@@ -7,6 +7,8 @@
 
 #include <atomic>
 
+#include "lmb_smem.h"
+
 struct lmb_lattice;
 
 // A context: one device and one stream.  It lives until its handle and every
@@ -209,6 +211,27 @@ static inline cudaError_t launch_chain(void (*k)(KArgs...), dim3 grid, dim3 bloc
     cfg.attrs = attr;
     cfg.numAttrs = 1;
     return cudaLaunchKernelEx(&cfg, k, args...);
+}
+
+// Raises kernel K's dynamic shared-memory limit on the current device to
+// `bytes` if it is lower (one limit per kernel: instantiations share a
+// function type, not a limit).  The kernel's static shared memory counts
+// against the default 48 KB too, so any size not granted yet is set.  CARVEOUT:
+// the share of the L1 array preferred as shared memory (none when negative).
+template <auto K, int CARVEOUT = -1>
+static cudaError_t raise_smem_limit(size_t bytes)
+{
+    static SmemLimit limit;
+    int device = 0;
+    const cudaError_t e = cudaGetDevice(&device);
+    if (e != cudaSuccess) return e;
+    const int rc = limit.raise(device, bytes, [](size_t b) {
+        cudaError_t s = cudaFuncSetAttribute(K, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)b);
+        if (s == cudaSuccess && CARVEOUT >= 0)
+            s = cudaFuncSetAttribute(K, cudaFuncAttributePreferredSharedMemoryCarveout, CARVEOUT);
+        return (int)s;
+    });
+    return rc == SmemLimit::BAD_DEVICE ? cudaErrorInvalidDevice : (cudaError_t)rc;
 }
 
 // Read-only view of a lattice for code outside the C ABI file (the .lm

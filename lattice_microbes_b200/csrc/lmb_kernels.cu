@@ -1070,23 +1070,12 @@ static size_t sweep_pp_smem(int BPS, int S, int NT)
     return (size_t)NT * (W * 4 + 8 + (size_t)S * 2 + (BPS == 1 ? W * 4 : 0));
 }
 
-// Raises kernel K's dynamic shared-memory limit once per device to the
-// largest size asked for so far (setting it on every launch costs host time).
-// One cache per kernel: instantiations share a function type, not a limit.
+// A sweep kernel's limit, and the whole unified L1 / shared array as shared
+// memory, so that as many blocks fit as the registers allow.
 template <auto K>
-static cudaError_t raise_smem_limit(size_t bytes)
+static cudaError_t raise_sweep_limit(size_t bytes)
 {
-    static size_t granted[64] = {0};
-    int dev = 0;
-    cudaGetDevice(&dev);
-    if (dev < 0 || dev >= 64) return cudaErrorInvalidDevice;
-    if (bytes <= 48 * 1024 || bytes <= granted[dev]) return cudaSuccess;
-    cudaError_t e = cudaFuncSetAttribute(K, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
-    // The whole unified L1 / shared array as shared memory, so that as many
-    // blocks fit as the registers allow.
-    if (e == cudaSuccess) e = cudaFuncSetAttribute(K, cudaFuncAttributePreferredSharedMemoryCarveout, 100);
-    if (e == cudaSuccess) granted[dev] = bytes;
-    return e;
+    return bytes <= 48 * 1024 ? cudaSuccess : raise_smem_limit<K, 100>(bytes);
 }
 
 cudaError_t launch_sweep(int bps, int slots, int dim, const uint32_t *src, uint32_t *dst, const uint8_t *sites,
@@ -1120,17 +1109,17 @@ cudaError_t launch_sweep(int bps, int slots, int dim, const uint32_t *src, uint3
     if (bps == BPS_ && slots == S_) {                                                                             \
         if (dim == 0) {                                                                                           \
             const size_t sm = sweep_pp_smem(BPS_, S_, SWEEP_THREADS);                                             \
-            if ((e = raise_smem_limit<sweep_pp_kernel<BPS_, S_, 0, SWEEP_THREADS>>(sm)) != cudaSuccess) return e;  \
+            if ((e = raise_sweep_limit<sweep_pp_kernel<BPS_, S_, 0, SWEEP_THREADS>>(sm)) != cudaSuccess) return e;  \
             e = launch_chain(sweep_pp_kernel<BPS_, S_, 0, SWEEP_THREADS>, grid, block, sm, stream, src, dst, sites, \
                              g, m, rs, list, cap, nullptr, 0u, pb_src, pb_dst);                                   \
         } else if (dim == 1) {                                                                                    \
             const size_t sm = sweep_pp_smem(BPS_, S_, YZ);                                                        \
-            if ((e = raise_smem_limit<sweep_pp_kernel<BPS_, S_, 1, YZ>>(sm)) != cudaSuccess) return e;            \
+            if ((e = raise_sweep_limit<sweep_pp_kernel<BPS_, S_, 1, YZ>>(sm)) != cudaSuccess) return e;            \
             e = launch_chain(sweep_pp_kernel<BPS_, S_, 1, YZ>, grid, block, sm, stream, src, dst, sites, g, m, rs, \
                              list, cap, nullptr, 0u, pb_src, pb_dst);                                             \
         } else {                                                                                                  \
             const size_t sm = sweep_pp_smem(BPS_, S_, YZ);                                                        \
-            if ((e = raise_smem_limit<sweep_pp_kernel<BPS_, S_, 2, YZ>>(sm)) != cudaSuccess) return e;            \
+            if ((e = raise_sweep_limit<sweep_pp_kernel<BPS_, S_, 2, YZ>>(sm)) != cudaSuccess) return e;            \
             e = launch_chain(sweep_pp_kernel<BPS_, S_, 2, YZ>, grid, block, sm, stream, src, dst, sites, g, m, rs, \
                              list, cap, rx_sites, rx_cap, pb_src, pb_dst);                                        \
         }                                                                                                         \

@@ -997,19 +997,6 @@ void list_fill_shape(const Geometry &g, TileShape &ts)
     ts.magic_q = list_magic(g.X / 4);
 }
 
-template <auto K>
-static cudaError_t list_smem_limit(size_t bytes)
-{
-    static size_t granted[64] = {0};
-    int dev = 0;
-    cudaGetDevice(&dev);
-    if (dev < 0 || dev >= 64) return cudaErrorInvalidDevice;
-    if (bytes <= granted[dev]) return cudaSuccess;
-    const cudaError_t e = cudaFuncSetAttribute(K, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
-    if (e == cudaSuccess) granted[dev] = bytes;
-    return e;
-}
-
 #define LIST_VARIANTS(X_)                                        \
     X_(1, 4) X_(1, 8) X_(1, 16) X_(4, 4) X_(4, 8) X_(4, 16)
 
@@ -1033,16 +1020,16 @@ cudaError_t launch_list(int bps, int slots, const uint32_t *src, uint32_t *dst, 
 #define LIST_LAUNCH(BPS_, S_)                                                                                     \
     if (bps == BPS_ && slots == S_) {                                                                             \
         if (small) {                                                                                              \
-            if ((e = list_smem_limit<list_step_kernel<BPS_, S_, 256, 4>>(smem)) != cudaSuccess) return e;          \
+            if ((e = raise_smem_limit<list_step_kernel<BPS_, S_, 256, 4>>(smem)) != cudaSuccess) return e;          \
             return launch_chain(list_step_kernel<BPS_, S_, 256, 4>, grid, dim3(256), smem, stream, src, dst, sites, \
                                 g, m, rs, queue, cap, ts, with_reaction, pb_src, pb_dst, (uint32_t)smem);          \
         }                                                                                                         \
         if (list_threads(ts.R, smem) == 1024u) {                                                                  \
-            if ((e = list_smem_limit<list_step_kernel<BPS_, S_, 1024, 1>>(smem)) != cudaSuccess) return e;         \
+            if ((e = raise_smem_limit<list_step_kernel<BPS_, S_, 1024, 1>>(smem)) != cudaSuccess) return e;         \
             return launch_chain(list_step_kernel<BPS_, S_, 1024, 1>, grid, dim3(1024), smem, stream, src, dst, sites, \
                                 g, m, rs, queue, cap, ts, with_reaction, pb_src, pb_dst, (uint32_t)smem);          \
         }                                                                                                         \
-        if ((e = list_smem_limit<list_step_kernel<BPS_, S_, 512, 2>>(smem)) != cudaSuccess) return e;              \
+        if ((e = raise_smem_limit<list_step_kernel<BPS_, S_, 512, 2>>(smem)) != cudaSuccess) return e;              \
         return launch_chain(list_step_kernel<BPS_, S_, 512, 2>, grid, dim3(512), smem, stream, src, dst, sites, g, m, \
                             rs, queue, cap, ts, with_reaction, pb_src, pb_dst, (uint32_t)smem);                    \
     }
@@ -1058,7 +1045,7 @@ cudaError_t launch_list_batch(int bps, int slots, const FusedJob *jobs, uint32_t
     count_launch();
 #define LIST_LAUNCH(BPS_, S_)                                                                                  \
     if (bps == BPS_ && slots == S_) {                                                                          \
-        if ((e = list_smem_limit<list_batch_kernel<BPS_, S_, 512, 2>>(smem)) != cudaSuccess) return e;          \
+        if ((e = raise_smem_limit<list_batch_kernel<BPS_, S_, 512, 2>>(smem)) != cudaSuccess) return e;          \
         return launch_chain(list_batch_kernel<BPS_, S_, 512, 2>, dim3(total_tiles), dim3(512), smem, stream, jobs, \
                             njobs, parity, (uint32_t)smem);                                                    \
     }
