@@ -30,10 +30,11 @@ def _run(ctx, spec, n, tile=(0, 0), lattice=None, records=1, tables=None):
     lat = Lattice(ctx, spec.X, spec.Y, spec.Z, spec.slots, spec.bytes_per_slot)
     lat.set_schedule(L.LMB_SCHEDULE_FUSED, *tile)
     lat.set_native(src, spec.sites)
-    step, rc = 0, 0
+    step, rc, split = 0, 0, 0
     for _ in range(records):
         rc, st, counts = lat.run_counts(model, 11, step, n, spec.ns, check=False)
         step += n
+        split += lat.tile_lists()[0]
         if rc:
             break
     out, _ = lat.get_native()
@@ -44,7 +45,7 @@ def _run(ctx, spec, n, tile=(0, 0), lattice=None, records=1, tables=None):
         assert np.array_equal(counts, oracle_counts(t, ref))
     lat.close()
     model.close()
-    return st_ref
+    return st_ref, split
 
 
 VARIANTS = [(4, 1), (8, 1), (16, 1), (4, 4), (8, 4), (16, 4)]
@@ -79,15 +80,19 @@ def test_crowded_corner_splits_its_tile(ctx, slots, bps):
             lat[(k // 4) * N + at[here]] |= sp[here] << np.uint32(8 * (k % 4))
         else:
             lat[k * N + at[here]] = sp[here]
-    _run(ctx, spec, 3, lattice=lat, records=2)
+    _, split = _run(ctx, spec, 3, lattice=lat, records=2)
+    assert split > 0
 
 
 @pytest.mark.parametrize("slots,bps", [(8, 1), (16, 4)])
 def test_more_reaction_candidates_than_listed(ctx, slots, bps):
     """Rates so high that most occupied sites may react in a timestep."""
-    spec = configs.random_problem(21, X=64, Y=16, Z=16, slots=slots, bytes_per_slot=bps, density=1.2, zeroth=False)
+    spec = configs.random_problem(21, X=64, Y=16, Z=16, slots=slots, bytes_per_slot=bps, density=0.6, zeroth=False)
     spec.K = spec.K * 40.0
-    st = _run(ctx, spec, 4, (16, 8))
+    # One timestep of two tiles, worked whole: one of them had more.
+    st, split = _run(ctx, spec, 1, (16, 8))
+    assert st.reactions > 2 * 512 and split == 0
+    st, _ = _run(ctx, spec, 4, (16, 8))
     assert st.reactions > 4 * 512
 
 
