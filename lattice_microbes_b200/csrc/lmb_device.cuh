@@ -17,8 +17,10 @@ namespace lmb {
 // before it in the stream has finished and its writes are visible (at once
 // when that kernel was not launched as part of a chain), then lets the next
 // kernel of the chain be launched, so that its blocks are scheduled while
-// this kernel's last blocks run instead of after them.  Nothing is read or
-// written before the wait.
+// this kernel's last blocks run instead of after them.  Before the wait a
+// kernel reads only what no kernel of the chain writes (the particle-list
+// kernels: site types, model tables, a batch's job table), and writes no
+// global memory.
 __device__ __forceinline__ void chain_enter()
 {
     asm volatile("griddepcontrol.wait;" ::: "memory");

@@ -499,11 +499,11 @@ struct ListTile {
             const uint32_t info = sh.rowinfo[r], gi = sh.rowbase[r] + xd;
             uint32_t ne = 0;
             if (pos >= (uint32_t)S) {
-                if (!(info & ROW_HALO)) overflow( 1u, gi, pos - (uint32_t)S, p);
+                if (!(info & ROW_HALO)) overflow(1u, gi, pos - (uint32_t)S, p);
             } else {
                 // A halo row matters for what it sends into the owned rows.
                 const bool lo = info & ROW_YL, up = info & ROW_YH;
-                    const uint32_t cy = hop(p, gi, pos, th[1], d, lo ? d : d - X, up ? d : d + X);
+                const uint32_t cy = hop(p, gi, pos, th[1], d, lo ? d : d - X, up ? d : d + X);
                 if (!((lo && cy != 2u) || (up && cy != 1u))) {
                     if (TWO) Q.put(d, pos, cy);
                     ne = (p << LIST_P) | (cy << LIST_C) | (d << LIST_L) | pos;
@@ -531,10 +531,10 @@ struct ListTile {
             if (!(info & (ROW_YL | ROW_YH))) {
                 const uint32_t pos = Q.place(l, k, c, d, d - X), gi = sh.rowbase[r] + x;
                 if (pos >= (uint32_t)S) {
-                    if (!(info & ROW_HALO)) overflow( 2u, gi, pos - (uint32_t)S, p);
+                    if (!(info & ROW_HALO)) overflow(2u, gi, pos - (uint32_t)S, p);
                 } else {
                     const bool lo = info & ROW_ZL, up = info & ROW_ZH;
-                            const uint32_t cz = hop(p, gi, pos, th[2], d, lo ? d : d - dz, up ? d : d + dz);
+                    const uint32_t cz = hop(p, gi, pos, th[2], d, lo ? d : d - dz, up ? d : d + dz);
                     if (!((lo && cz != 2u) || (up && cz != 1u))) {
                         if (TWO) P.put(d, pos, cz);
                         ne = (p << LIST_P) | (cz << LIST_C) | (d << LIST_L) | pos;
@@ -567,7 +567,7 @@ struct ListTile {
             if (!(info & ROW_HALO)) {
                 const uint32_t pos = P.place(l, k, c, d, d - dz), gi = sh.rowbase[r] + x;
                 if (pos >= (uint32_t)S) {
-                    overflow( 3u, gi, pos - (uint32_t)S, p);
+                    overflow(3u, gi, pos - (uint32_t)S, p);
                 } else {
                     ne = e;
                     if (BPS == 1)

@@ -109,10 +109,12 @@ struct lmb_server {
     uint64_t completed;
 };
 
-// Device bytes a resident solve holds: two particle buffers, site types, the
-// overflow queue and run state (lmb_lattice_create), the reaction site list
-// of the per-phase schedule (N / 8 + 4096 entries of 8 bytes), and the model tables
-// (lmb_model_create).
+// Device bytes a resident solve is counted with: two particle buffers, site
+// types, the overflow queue and run state (lmb_lattice_create), the reaction
+// site list of the per-phase schedule (N / 8 + 4096 entries of 8 bytes), and
+// the model tables (lmb_model_create).  Particle-list tiles keep plane bounds
+// (at most N / 4 bytes) instead of that list; a large solve on the per-phase
+// kernels holds both, the bounds not counted.
 static uint64_t request_bytes(const lmb_server *s, const Request &r)
 {
     const uint64_t N = (uint64_t)r.X * r.Y * r.Z;
