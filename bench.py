@@ -365,8 +365,10 @@ def ncu_traffic_per_launch(workload, kernel):
     summary (profiles/traffic.json), if any."""
     try:
         d = json.load(open(os.path.join(ROOT, "profiles", "traffic.json")))
-        e = d.get(workload) or {}
-        return e.get("kernel_dram_bytes_per_launch") if e.get("kernel", "").startswith(kernel) else None
+        for e in d.get(workload, []):
+            if e["kernel"].startswith(kernel):
+                return e["kernel_dram_bytes_per_launch"]
+        return None
     except Exception:
         return None
 
@@ -506,10 +508,12 @@ def run_ours(a):
                 if sched[0] == LL.LMB_SCHEDULE_CLUSTER else
                 "fused_grid_kernel (every timestep of the run in one launch; per timestep)"
                 if sched[0] == LL.LMB_SCHEDULE_GRID else
-                "fused_step_kernel (x, y, z sweeps + reaction + overflow, one timestep)")
+                "list_step_kernel (x, y, z sweeps + reaction + overflow by particle, one timestep)")
         launch_ms = phases["fused_step"]["ms_per_launch"]
         alg_bytes = N * B_STEP                 # site-steps per launch x per-site-step bytes
-        own_bytes = N * B_SWEEP                # its own dataflow: read slots + site type, write slots
+        # Its own dataflow is what its particles take (particle-list tiles) or
+        # what crosses between runs (resident forms): the ncu DRAM traffic, when recorded.
+        own_bytes = ncu_traffic_per_launch(a.workload, kern.split()[0])
     else:
         kern = "sweep_pp_kernel (x, y, z hop sweeps by particle)"
         sweep_share = float(phase_ms[:3].sum()) / total_ms
@@ -591,16 +595,17 @@ def run_ours(a):
                 "peak": peak,
                 "unit": "GB/s",
                 "frac": achieved / peak,
-                "traffic": ncu_traffic_per_launch(a.workload, "fused_step_kernel" if phase_n[5] > 0 else "sweep"),
+                "traffic": ncu_traffic_per_launch(a.workload, kern.split()[0] if phase_n[5] > 0 else "sweep"),
                 "kernel": kern,
                 "ms_per_launch": launch_ms,
                 "algorithmic_bytes_per_launch": alg_bytes,
                 "own_dataflow_bytes_per_launch": own_bytes,
-                "own_dataflow_frac": own_bytes / (launch_ms / 1e3) / 1e9 / peak,
+                "own_dataflow_frac": None if own_bytes is None else own_bytes / (launch_ms / 1e3) / 1e9 / peak,
                 "peak_kind": peak_kind,
                 "note": (("achieved = N x B_step (reference-schedule bytes of a site-step) per fused launch / "
-                          "launch time; own_dataflow_frac counts the fused kernel's single read and write of the "
-                          "lattice" if phase_n[5] > 0 else
+                          "launch time, which a timestep by particle does not move: frac is a rate in those bytes, "
+                          "not HBM use; own_dataflow_frac (ncu DRAM bytes per launch, where recorded) is, and the "
+                          "launches are bound by instruction issue and latency" if phase_n[5] > 0 else
                           "achieved = N x B_sweep (reference-schedule bytes of a site's sweep) per sweep launch / "
                           "sweep launch time; the sweeps keep per-segment plane bounds and move only the word "
                           "planes that can hold particles, so own_dataflow_frac (ncu DRAM bytes per launch) is far "
