@@ -928,7 +928,11 @@ int lmb::lattice_view(const lmb_lattice *l, LatticeView *v)
     return LMB_OK;
 }
 
-bool lmb::lattice_by_particle(const lmb_lattice *l) { return l->schedule == LMB_SCHEDULE_FUSED && l->tile.list_smem != 0; }
+bool lmb::lattice_by_particle(const lmb_lattice *l, uint32_t number_species)
+{
+    return l->schedule == LMB_SCHEDULE_FUSED && l->tile.list_smem != 0 &&
+           (l->bps == 1 || number_species <= LIST_MAX_SPECIES);
+}
 
 extern "C" int lmb_lattice_device_buffers(lmb_lattice *l, void **particles, void **sites)
 {
@@ -985,7 +989,10 @@ static uint32_t *plane_bounds(lmb_lattice *l, int b) { return l->pb ? l->pb + (s
 // model's species ids, the dense fused kernel where they do not, and the
 // per-phase kernels for PHASES, for a tile that only the particle-list
 // kernel could hold, and for a lattice of its own schedule whose particles
-// crowd (note_splits).
+// crowd (note_splits).  A smaller dense tile is not looked for: IntLattice-8
+// with 5,000 species, per-phase / dense in its default tile, us per timestep:
+// 128 x 64 x 64 at 0.005 particles per site 28 / 164, at 0.3 49 / 341, 64^3
+// at 0.005 20 / 41.
 enum StepKind { STEP_LIST, STEP_DENSE, STEP_PHASES };
 
 static StepKind step_kind(const lmb_lattice *l, const lmb_model *m)
@@ -993,6 +1000,20 @@ static StepKind step_kind(const lmb_lattice *l, const lmb_model *m)
     if (l->schedule != LMB_SCHEDULE_FUSED || (l->own_schedule && l->crowded)) return STEP_PHASES;
     if (l->tile.list_smem && (l->bps == 1 || m->ns <= LIST_MAX_SPECIES)) return STEP_LIST;
     return l->tile.dense ? STEP_DENSE : STEP_PHASES;
+}
+
+// The kernels of a run, with the device memory they need.  A crowded lattice
+// that finds none for the per-phase kernels stays on its tiles.
+static int prepare_step_kind(lmb_lattice *l, const lmb_model *m, StepKind &kind)
+{
+    kind = step_kind(l, m);
+    if (kind != STEP_PHASES) return LMB_OK;
+    const int rc = ensure_phase_buffers(l);
+    if (rc == LMB_OK || !l->crowded) return rc;
+    cudaGetLastError();
+    l->crowded = false;
+    kind = step_kind(l, m);
+    return kind == STEP_PHASES ? rc : LMB_OK;
 }
 
 // One fused launch (list or dense form), from the current buffer.
@@ -1169,8 +1190,8 @@ static int run_async(lmb_lattice *l, const lmb_model *mc, uint32_t seed, uint32_
     if (rc) return rc;
     if (device_check && m->nr > 0) l->run_species = std::max(l->run_species, m->ns);
     follow_density(l);
-    const StepKind kind = step_kind(l, m);
-    if (kind == STEP_PHASES && (rc = ensure_phase_buffers(l)) != LMB_OK) return rc;
+    StepKind kind;
+    if ((rc = prepare_step_kind(l, m, kind)) != LMB_OK) return rc;
     const bool counting = count_ns != ~0u;
     // The fused kernels count in their last launch when their shared memory
     // holds the histogram; otherwise one pass over the final lattice follows
@@ -1352,8 +1373,8 @@ extern "C" int lmb_run_profiled(lmb_lattice *l, const lmb_model *mc, uint32_t se
     int rc = validate_for_model(l, m);
     if (rc) return rc;
     follow_density(l);
-    const StepKind kind = step_kind(l, m);
-    if (kind == STEP_PHASES && (rc = ensure_phase_buffers(l)) != LMB_OK) return rc;
+    StepKind kind;
+    if ((rc = prepare_step_kind(l, m, kind)) != LMB_OK) return rc;
     CK(launch_begin_run(l->rs, seed, first, n, (uint32_t)mode, c->stream));
     CK(reset_plane_bounds(l, m, c->stream));
     std::vector<cudaEvent_t> ev((size_t)n * 12);

@@ -246,7 +246,8 @@ struct LatticeView {
 };
 int lattice_view(const lmb_lattice *lattice, LatticeView *view);
 
-// The lattice's fused plan is one of particle-list tiles.
-bool lattice_by_particle(const lmb_lattice *lattice);
+// The lattice's fused plan is one of particle-list tiles, for models of this
+// many species.
+bool lattice_by_particle(const lmb_lattice *lattice, uint32_t number_species);
 
 }  // namespace lmb

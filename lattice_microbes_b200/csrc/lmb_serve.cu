@@ -306,7 +306,7 @@ static int admit(lmb_server *s)
         int rc = lmb_model_create(c, &d, a.req.X, a.req.Y, a.req.Z, &a.model);
         if (rc == LMB_OK) rc = lmb_lattice_create(c, a.req.X, a.req.Y, a.req.Z, s->slots, s->bps, &a.lat);
         if (rc == LMB_OK) rc = lmb_lattice_set_native(a.lat, a.req.particles.data(), a.req.sites.data());
-        if (rc == LMB_OK && a.solo && !lmb::lattice_by_particle(a.lat)) {
+        if (rc == LMB_OK && a.solo && !lmb::lattice_by_particle(a.lat, a.req.ns)) {
             const double density = (double)count_particles(a.req.particles, s->bps) / (double)nsites;
             if (density >= DENSE_PARTICLES_PER_SITE) rc = lmb_lattice_set_schedule(a.lat, LMB_SCHEDULE_PHASES, 0, 0);
         }

@@ -205,3 +205,35 @@ def test_server_isolates_a_failing_solve(ctx):
         assert info.stats.status == 0
         _, _, ref, _ = solo(ctx, spec, seed, 0, r.timesteps)
         assert np.array_equal(lat, ref)
+
+
+def test_large_solve_of_many_species_runs_per_phase(ctx):
+    """A dense IntLattice solve whose species ids do not fit a particle-list
+    entry: served with the per-phase kernels (several launches a timestep),
+    as such solves are without list tiles."""
+    from lattice_microbes_b200.solver import Server, kernel_launches
+    few = configs.random_problem(91, X=64, Y=64, Z=32, slots=8, bytes_per_slot=4, ns=3, nst=1, nr=3, density=0.1,
+                                 zeroth=False)
+    ns = 4100
+    ids = np.array([0, 17, 4097, 4100], dtype=np.uint32)
+    spec = configs.ModelSpec(**{**few.__dict__, "ns": ns, "S": np.zeros((ns, few.nr), np.int32),
+                                "D": np.zeros((ns, few.nr), np.uint32), "DF": np.zeros((1, 1, ns)),
+                                "lattice": ids[few.lattice]})
+    for s in range(3):
+        spec.S[ids[s + 1] - 1], spec.D[ids[s + 1] - 1] = few.S[s], few.D[s]
+        spec.DF[:, :, ids[s + 1] - 1] = few.DF[:, :, s]
+    server = Server(ctx, slots=8, bytes_per_slot=4, chunk_timesteps=8)
+    server.submit(1, spec, 5, 16)
+    before = kernel_launches()
+    while True:
+        server.step()
+        got = server.pop_result()
+        if got:
+            break
+    assert kernel_launches() - before >= 4 * 16
+    info, words, _ = got
+    assert info.stats.status == 0
+    ref, rc, _ = oracle_run(oracle_tables(few), few.lattice, few.sites, 5, 0, 16)
+    assert rc == 0
+    assert np.array_equal(words, ids[ref])
+    server.close()
