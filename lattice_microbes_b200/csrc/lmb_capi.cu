@@ -1992,6 +1992,7 @@ extern "C" int lmb_batch_autotune(lmb_batch *b, const uint32_t *seeds, uint32_t 
     if (b->pending) return LMB_E_STATE;
     lmb_ctx *c = b->ctx;
     CK(cudaSetDevice(c->device));
+    batch_prepare(b);  // contents counted (a member that cannot run shows in the trials)
     const uint32_t count = (uint32_t)b->lats.size();
     std::vector<size_t> off(count);
     size_t total = 0;
@@ -2019,9 +2020,19 @@ extern "C" int lmb_batch_autotune(lmb_batch *b, const uint32_t *seeds, uint32_t 
                             cudaMemcpyDeviceToDevice, c->stream);
         }
     };
+    // What one tile shape could not hold sizes no other's lists.
+    std::vector<std::pair<float, float>> figures;
+    for (const lmb_lattice *l : b->lats) figures.push_back({l->density, l->crowd});
+    auto restore_figures = [&]() {
+        for (uint32_t j = 0; j < count; j++) {
+            b->lats[j]->density = figures[j].first;
+            b->lats[j]->crowd = figures[j].second;
+        }
+    };
     // Time of one trial (the better of two), or a large value when it fails.
     auto trial = [&]() -> float {
         float best = 1e30f;
+        restore_figures();
         for (int rep = 0; rep < 2; rep++) {
             restore();
             cudaEventRecord(e0, c->stream);
@@ -2049,6 +2060,7 @@ extern "C" int lmb_batch_autotune(lmb_batch *b, const uint32_t *seeds, uint32_t 
     for (const auto &key : order) {
         const std::vector<uint32_t> &members = classes[key];
         const Geometry g = b->lats[members[0]]->g;
+        restore_figures();
         TileShape keep = b->tiles[members[0]];
         for (uint32_t Ty : cands)
             for (uint32_t Tz : cands) {
@@ -2059,6 +2071,7 @@ extern "C" int lmb_batch_autotune(lmb_batch *b, const uint32_t *seeds, uint32_t 
                 if (t.Ty == keep.Ty && t.Tz == keep.Tz) continue;
                 for (uint32_t j : members) b->tiles[j] = t;
                 const float ms = trial();
+                restore_figures();
                 if (ms < best) {
                     best = ms;
                     keep = t;
@@ -2068,6 +2081,7 @@ extern "C" int lmb_batch_autotune(lmb_batch *b, const uint32_t *seeds, uint32_t 
         b->tuned[key] = {keep.Ty, keep.Tz};
     }
     restore();
+    restore_figures();
     const cudaError_t e = cudaStreamSynchronize(c->stream);
     cudaFree(save);
     cudaEventDestroy(e0);

@@ -103,3 +103,39 @@ def test_batch_autotune_keeps_state_and_results(gpu):
         lat.close()
         m.close()
     ctx.close()
+
+
+def test_batch_autotune_leaves_the_lattices_figures(gpu):
+    """Members whose particles crowd into some z planes: tiles are split in
+    the trials, and the lists of the members' own plans are still sized for
+    the particles they hold, not for what a trial's tile could not."""
+    from lattice_microbes_b200 import _lib as L
+    from lattice_microbes_b200.solver import Batch, Context
+    ctx = Context(0)
+    specs, rng = [], np.random.default_rng(8)
+    for k in range(3):
+        s = configs.random_problem(300 + k, X=32, Y=32, Z=32, slots=8, bytes_per_slot=1, density=0.0, nst=1, qmax=0.02,
+                                   zeroth=False)
+        lat = np.zeros_like(s.lattice)
+        for q in range(4):
+            at = np.arange(5 * 1024)
+            lat[at] |= rng.integers(1, s.ns + 1, at.size).astype(np.uint32) << np.uint32(8 * q)
+        s.lattice = lat
+        specs.append(s)
+    seeds = [5, 6, 7]
+    pairs = [_make(ctx, s) for s in specs]
+    batch = Batch(ctx, [p[0] for p in pairs], [p[1] for p in pairs])
+    batch.autotune(seeds, 0, 4)
+    mean = 4 * 5 / 32
+    for lat, _ in pairs:
+        lat.set_schedule(L.LMB_SCHEDULE_FUSED)
+        assert lat.tile_lists()[1] == pytest.approx(mean)
+    rc, _ = batch.run(seeds, 0, 6)
+    assert rc == 0
+    assert max(lat.tile_lists()[0] for lat, _ in pairs) > 0
+    for (lat, m), spec, seed in zip(pairs, specs, seeds):
+        assert np.array_equal(lat.get_native()[0], oracle_run(oracle_tables(spec), spec.lattice, spec.sites, seed, 0, 6)[0])
+        lat.close()
+        m.close()
+    batch.close()
+    ctx.close()
