@@ -43,7 +43,8 @@ extern "C" {
 /* Timestep schedules.  FUSED runs the x, y, z sweeps and the reaction of a
  * tile of Ty x Tz full x-rows in shared memory, one launch per timestep (the
  * tile's particles in a list, whose length follows the lattice's density;
- * with Ty = Tz = 0 the tile does too);
+ * with Ty = Tz = 0 the tile does too, and a lattice that was never given a
+ * schedule runs the PHASES kernels while its particles crowd into few tiles);
  * PHASES launches one kernel per sweep, the reaction and the overflow pass
  * (the reference's schedule, MpdRdmeSolver.cu:1011-1090); CLUSTER, for small
  * lattices, holds the whole lattice in the shared memory of one thread-block
